@@ -30,10 +30,14 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
                   "-I" + str(ROOT / "include")]
 
-CU_SOURCES = ["runtime.cu", "spmv.cu", "sell.cu", "sparse_ops.cu", "reduce.cu", "cg.cu", "cg_mixed.cu", "cg_plain.cu",
-              "cg_coop.cu", "cg_cluster.cu", "lincomb.cu"]
+# (cg_mixed.cu is compiled once per CTA size and inner value type: one
+# translation unit of all its kernels takes ten minutes of ptxas)
+MIXED_UNITS = [(t, mi) for t in (256, 512, 1024) for mi in ("float", "__nv_bfloat16")]
+CU_SOURCES = ["runtime.cu", "spmv.cu", "sell.cu", "sparse_ops.cu", "reduce.cu", "cg.cu", "cg_plain.cu",
+              "cg_coop.cu", "cg_cluster.cu", "cg_resident.cu", "lincomb.cu"]
 HEADERS = ["common.cuh", "objects.h", "spmv_dev.cuh", "cg_dev.cuh", "tma.cuh", "cg_smem.cuh", "cg_grid.cuh",
-           "grid_sync.cuh", "cg_compact.cuh", "cg_plain.cuh", "cg_cluster.cuh"]
+           "grid_sync.cuh", "cg_compact.cuh", "cg_plain.cuh", "cg_cluster.cuh",
+           "cg_resident.cuh", "tagged.cuh"]
 
 
 def _stale(target: Path, deps: list[Path]) -> bool:
@@ -70,13 +74,16 @@ def build_cuda(verbose: bool = False, ptxas_info: bool = False) -> Path:
     LIB.mkdir(exist_ok=True)
     jobs = []
     objs = []
-    for src in CU_SOURCES:
+    units = [("cg_mixed.cu", f"cg_mixed.{t}.{mi}", [f"-DCMCG_MIXED_T={t}", f"-DCMCG_MIXED_MI={mi}"])
+             for t, mi in MIXED_UNITS]   # (the slowest first)
+    units += [(src, src, []) for src in CU_SOURCES]
+    for src, name, defs in units:
         s = CSRC / src
-        o = OBJ / (src + ".o")
+        o = OBJ / (name + ".o")
         objs.append(o)
         if _stale(o, _local_deps(s)) or ptxas_info:
             extra = ["-Xptxas", "-v"] if ptxas_info else []
-            jobs.append([NVCC] + NVFLAGS + extra + ["-c", str(s), "-o", str(o)])
+            jobs.append([NVCC] + NVFLAGS + defs + extra + ["-c", str(s), "-o", str(o)])
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         list(ex.map(_run, jobs))
     so = LIB / "libcumat_cg.so"

@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "cg_grid.cuh"
 #include "cg_plain.cuh"
+#include "cg_resident.cuh"
 #include "objects.h"
 
 namespace cmcg {
@@ -1329,21 +1330,6 @@ __global__ void __launch_bounds__(kTile, kGridCtasPerSm) k_grid_pupdate(SolveArg
 // ---------------------------------------------------------------------------
 
 template <typename MI, typename MO>
-struct GMixArgs {
-    SolveArgs<float, MI> g;   // plan, segments, inner vectors r/p/q (FP32), state; g.m = scaled inner values
-    MatArgs<MO> mo;           // outer values (unscaled) in the sliced layout
-    const double* s;          // [mb][rows]
-    const double* b64;
-    double* x64;
-    float* xh;
-    double* p1;               // FP64 partials of the residual replacement
-    double* p2;
-    double outer_tol;
-    int32_t max_updates;
-    float delta;
-};
-
-template <typename MI, typename MO>
 __global__ void __launch_bounds__(kTile, kGridCtasPerSm) k_gmix_init(GMixArgs<MI, MO> m) {
     const SolveArgs<float, MI>& a = m.g;
     __shared__ double red[2 * (kTile / 32)];
@@ -1463,28 +1449,6 @@ __global__ void __launch_bounds__(kTile, kGridCtasPerSm) k_gmix_spmv(GMixArgs<MI
             }
         }
     }
-}
-
-// Condition probe of BF16 inner values (grid path). CG's residual contracts
-// at least as fast as its bound for the scaled system's condition number
-// kappa, so the rate rho observed over the first kCondProbe iterations gives
-// a lower estimate kappa >= ((1 + rho) / (1 - rho))^2. Refinement through an
-// inner system rounded to BF16 (unit roundoff 2^-8) needs kappa * 2^-8 well
-// below 1; above kBf16CondLimit the instance stops with BREAKDOWN, and the
-// FP32 fallback solves it, instead of the progress guard's thousands of
-// iterations later. ratio = |r_k|^2 / |r_0|^2 of the first cycle.
-constexpr int32_t kCondProbe = 64;
-constexpr float kBf16CondLimit = 256.0f;
-// The same decision at every replacement: the inner recursion claimed |r|^2
-// down by delta^2 since the last one, the true FP64 residual is down by about
-// (delta + u kappa)^2; a true ratio above kBf16Lag delta^2 means the BF16
-// rounding term dominates, and the cycles to come will crawl.
-constexpr double kBf16Lag = 10.0;
-__device__ __forceinline__ bool bf16_condition_ok(float ratio, int32_t k) {
-    if (!(ratio < 1.0f)) return false;   // no contraction at all (or NaN)
-    const float rho = powf(ratio, 0.5f / static_cast<float>(k));
-    const float s = (1.0f + rho) / (1.0f - rho);
-    return s * s <= kBf16CondLimit;
 }
 
 // xh += alpha p_k, r -= alpha q, |r|^2 -> replacement decision or beta
@@ -1781,6 +1745,9 @@ struct cmcg_solver_s {
     int coop = 1;
     // cluster solve of the grid path where it applies (CUMAT_CG_CLUSTER=0 disables)
     bool cluster = true;
+    // chip-resident solve of the grid path where it applies (CUMAT_CG_RESIDENT=0 disables)
+    bool resident = true;
+    void* res_ws = nullptr;   size_t res_ws_bytes = 0;
     // grid path: the product forms p_k (-1: by the batch's vector bytes against
     // L2, see fuse_p_update; 0 / 1: CUMAT_CG_FUSE)
     int fuse_p = -1;
@@ -2564,6 +2531,69 @@ cmcg_status run_grid(cmcg_solver s, SolveArgs<VT, MT>& a) {
     return CMCG_OK;
 }
 
+// The dynamic shared memory a resident CTA may use (its static scratch is below 2 KB).
+cmcg_status resident_smem_limit(cmcg_ctx ctx, size_t* bytes) {
+    int optin = 0;
+    CMCG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    *bytes = static_cast<size_t>(std::max(0, optin - 2048));
+    return CMCG_OK;
+}
+
+// The geometry of a chip-resident solve of the solver's one system on the
+// grid plan; *ok = false where it does not apply (see resident_plan). The
+// offsets come from the host copy of the diagonal plan.
+cmcg_status resident_geom(cmcg_solver s, int32_t ob, size_t val_bytes, size_t vec_bytes, ResidentGeom* g, bool* ok) {
+    *ok = false;
+    cmcg_pattern p = s->A->pat;
+    const DiaPlan& D = p->dia;
+    if (!s->resident || !s->graph_loop || s->n_sys != 1 || ob != 1 || !D.ok || (D.max_nd != 5 && D.max_nd != 7))
+        return CMCG_OK;
+    size_t limit = 0;
+    CMCG_TRY(resident_smem_limit(p->ctx, &limit));
+    *ok = resident_plan(*g, p->rows, s->grid_ctas, D.max_nd, D.off0, p->ctx->sm_count, val_bytes, vec_bytes, limit);
+    return CMCG_OK;
+}
+
+// The grid path's loop of one stencil system whose vectors fit the chip, as
+// one cooperative launch (cg_resident.cu) after the grid path's init kernels.
+// *done = false leaves the solve to the graph loop. Faster wherever it fits, us
+// per iteration here against the graph loop: FP32 Poisson 400^2 7.2 / 21.2, 1024^2
+// 10.6 / 26.3, 1023^2 14.7 / 31.2; 3-D 7-point 64^3 9.3 / 22.5, 96^3 20.7 / 28.4;
+// FP64 300^2 9.5 / 22.0, 720^2 12.8 / 31.5.
+template <typename VT, typename MT, int FMT>
+cmcg_status run_resident(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
+    *done = false;
+    if (FMT != CMCG_CSR || !s->resident || s->n_sys != 1 || a.ob != 1) return CMCG_OK;
+    cmcg_pattern p = s->A->pat;
+    cmcg_ctx ctx = p->ctx;
+    cudaStream_t st = ctx->stream;
+    bool dia = false, ok = false;
+    CMCG_TRY(ensure_dia_plain(s, &dia));
+    if (!dia) return CMCG_OK;
+    const DiaPlan& D = p->dia;
+    ResidentGeom g;
+    CMCG_TRY(resident_geom(s, a.ob, sizeof(MT), sizeof(VT), &g, &ok));
+    if (!ok) return CMCG_OK;
+    const int64_t items = a.n_seg;
+    CMCG_TRY(ensure_buffer(&s->part_ws, &s->part_ws_bytes, 2 * sizeof(VT) * static_cast<size_t>(items) + 64));
+    CMCG_TRY(ensure_buffer(&s->res_ws, &s->res_ws_bytes, resident_ws_bytes(g, sizeof(VT))));
+    a.part1 = static_cast<VT*>(s->part_ws);
+    a.part2 = a.part1 + items;
+    a.dia = DiaArgs<MT>{static_cast<const MT*>(s->dia_plain), s->dia_plain_stride, D.d_sys_base, D.d_sys_off, nullptr,
+                        s->A->batches};
+    CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 3 * sizeof(int32_t), st));
+    k_grid_init<VT, MT, FMT><<<s->grid_ctas, kTile, 0, st>>>(a);
+    k_grid_init2<VT, MT, FMT><<<s->grid_ctas, kTile, 0, st>>>(a);
+    count_launch(2);
+    CMCG_CHECK_LAUNCH();
+    CMCG_TRY((resident_cg_launch<VT, MT>(a, g, D.max_nd, s->res_ws, ctx->d_err, st, done)));
+    if (*done) count_launch();
+    if (log_on(2))
+        log_msg(2, "resident solve%s: %d CTAs, %d of %d diagonals in shared memory", *done ? "" : " not launched", g.ctas,
+                g.smem_diags, D.max_nd);
+    return CMCG_OK;
+}
+
 // One thread-block cluster per instance (cg_cluster.cu), when the largest
 // system has more than kClusterMinRows rows yet its vectors fit the shared
 // memory of at most kClusterMaxCtas CTAs, and all instances' clusters can be
@@ -2706,6 +2736,7 @@ cmcg_status solve_t(cmcg_solver s, const VT* b, int32_t b_b, const VT* guess, VT
         bool done = false;
         CMCG_TRY((run_cluster<VT, MT, FMT>(s, a, &done)));
         if (!done) CMCG_TRY((run_coop<VT, MT, FMT>(s, a, w + 4 * nv, &done)));
+        if (!done) CMCG_TRY((run_resident<VT, MT, FMT>(s, a, &done)));
         if (!done) CMCG_TRY((run_grid<VT, MT, FMT>(s, a)));
         const int fb = (n_inst + 255) / 256;
         k_finalize<<<fb, 256, 0, ctx->stream>>>(s->st, n_inst);
@@ -3067,6 +3098,20 @@ cmcg_status refined_grid_mixed(cmcg_solver s, cmcg_matrix Ao, const double* b, i
     k_gmix_init<MI, MO><<<grid, kTile, 0, st>>>(m);
     count_launch();
     CMCG_CHECK_LAUNCH();
+    // one stencil system whose vectors fit the chip: the loop in one launch (us per
+    // iteration against the graph loop: 200^2 6.3 / 20.8, 1024^2 10.0 / 33.0, 64^3
+    // 9.9 / 30.3, 96^3 20.0 / 34.5)
+    bool resident = false;
+    if (nd > 0) {
+        ResidentGeom rg;
+        bool ok = false;
+        CMCG_TRY(resident_geom(s, ob, sizeof(MI), sizeof(float), &rg, &ok));
+        if (ok) {
+            CMCG_TRY(ensure_buffer(&s->res_ws, &s->res_ws_bytes, resident_ws_bytes(rg, sizeof(float))));
+            CMCG_TRY((resident_mixed_launch<MI, MO>(m, rg, nd, s->res_ws, ctx->d_err, st, &resident)));
+            if (resident) count_launch();
+        }
+    }
     // one iteration's kernels on stream t
     const auto iteration = [&](cudaStream_t t) {
         const auto product = [&](auto fuse) {
@@ -3082,7 +3127,9 @@ cmcg_status refined_grid_mixed(cmcg_solver s, cmcg_matrix Ao, const double* b, i
         k_gmix_residual<MI, MO, false><<<grid, kTile, 0, t>>>(m);
         if (!fused) k_gmix_pupdate<MI, MO><<<grid, kTile, 0, t>>>(m);
     };
-    if (!s->graph_loop) {
+    if (resident) {
+        // (the closing fold and residual below take what a breakdown left)
+    } else if (!s->graph_loop) {
         CMCG_TRY(host_loop(st, m.g.active, m.g.loop_cap, fused ? 5 : 6, [&] {
             iteration(st);
             k_loop_step<<<1, 1, 0, st>>>(m.g.loops);
@@ -3166,6 +3213,7 @@ cmcg_status cmcg_cg_create(cmcg_matrix A, int32_t precond, cmcg_solver* out) {
     if (const char* e = std::getenv("CUMAT_CG_SMALL")) s->mix_small = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_COOP")) s->coop = std::max(0, std::min(2, std::atoi(e)));
     if (const char* e = std::getenv("CUMAT_CG_CLUSTER")) s->cluster = std::atoi(e) != 0;
+    if (const char* e = std::getenv("CUMAT_CG_RESIDENT")) s->resident = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_FUSE")) s->fuse_p = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_GRAPH")) s->graph_loop = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_BF16_FALLBACK")) s->bf16_fallback = std::atoi(e) != 0;
@@ -3200,7 +3248,7 @@ cmcg_status cmcg_cg_destroy(cmcg_solver s) {
                     static_cast<void*>(s->d_seg_t1), static_cast<void*>(s->d_seg_sys), static_cast<void*>(s->d_cta_seg0),
                     static_cast<void*>(s->d_sys_seg0), static_cast<void*>(s->d_cseg_t0), static_cast<void*>(s->d_cseg_t1),
                     static_cast<void*>(s->d_cseg_sys), static_cast<void*>(s->d_ccta_seg0),
-                    static_cast<void*>(s->d_csys_seg0), s->dinv[0], s->dinv[1], s->vec_ws, s->ref_ws, s->part_ws,
+                    static_cast<void*>(s->d_csys_seg0), s->dinv[0], s->dinv[1], s->vec_ws, s->ref_ws, s->part_ws, s->res_ws,
                     s->st_ws, static_cast<void*>(s->counters), s->mix_vals, static_cast<void*>(s->mix_s),
                     s->dia_vals, s->dia_plain})
         dev_free(p);

@@ -192,11 +192,19 @@ struct MixArgs {
 constexpr int kMixSmallRows = kSmemNK * 512;
 constexpr int kMixTinyRows = kSmemNK * 256;
 
-// Launches k_mixed_fast (cg_mixed.cu) with `threads` (1024, 512 or 256) threads per
-// CTA and `smem` bytes of dynamic shared memory: nd = 0 sliced layout, nd = 5
-// or 7 diagonal layout.
+// Launches k_mixed_fast (cg_mixed.cu, one translation unit per T and MI) with
+// `threads` (1024, 512 or 256) threads per CTA and `smem` bytes of dynamic
+// shared memory: nd = 0 sliced layout, nd = 5 or 7 diagonal layout.
+template <typename MI, typename MO, int T>
+cmcg_status launch_mixed_t(const MixArgs<MI, MO>& m, int nmax, size_t smem, int nd, int grid, cudaStream_t stream);
+
 template <typename MI, typename MO>
 cmcg_status launch_mixed_fast(const MixArgs<MI, MO>& m, int threads, int nmax, size_t smem, int nd, int grid,
-                              cudaStream_t stream);
+                              cudaStream_t stream) {
+    if (threads == 256) return launch_mixed_t<MI, MO, 256>(m, nmax, smem, nd, grid, stream);
+    if (threads == 512) return launch_mixed_t<MI, MO, 512>(m, nmax, smem, nd, grid, stream);
+    if (threads == kSmemThreads) return launch_mixed_t<MI, MO, kSmemThreads>(m, nmax, smem, nd, grid, stream);
+    return fail(CMCG_ERR_INVALID_ARGUMENT, "unsupported CTA size");
+}
 
 }  // namespace cmcg

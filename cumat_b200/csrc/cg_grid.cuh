@@ -264,6 +264,44 @@ __device__ __forceinline__ void seg_rows_vec(int r0, int r1, const void* const (
     for (int b_ = 0; b_ < (a).ob; ++b_)                                          \
         for (int seg_ = (a).cta_seg0[blockIdx.x]; seg_ < (a).cta_seg0[blockIdx.x + 1]; ++seg_)
 
+// Arguments of the grid path's mixed solve.
+template <typename MI, typename MO>
+struct GMixArgs {
+    SolveArgs<float, MI> g;   // plan, segments, inner vectors r/p/q (FP32), state; g.m = scaled inner values
+    MatArgs<MO> mo;           // outer values (unscaled) in the sliced layout
+    const double* s;          // [mb][rows]
+    const double* b64;
+    double* x64;
+    float* xh;
+    double* p1;               // FP64 partials of the residual replacement
+    double* p2;
+    double outer_tol;
+    int32_t max_updates;
+    float delta;
+};
+
+// Condition probe of BF16 inner values (grid path). CG's residual contracts
+// at least as fast as its bound for the scaled system's condition number
+// kappa, so the rate rho observed over the first kCondProbe iterations gives
+// a lower estimate kappa >= ((1 + rho) / (1 - rho))^2. Refinement through an
+// inner system rounded to BF16 (unit roundoff 2^-8) needs kappa * 2^-8 well
+// below 1; above kBf16CondLimit the instance stops with BREAKDOWN, and the
+// FP32 fallback solves it, instead of the progress guard's thousands of
+// iterations later. ratio = |r_k|^2 / |r_0|^2 of the first cycle.
+constexpr int32_t kCondProbe = 64;
+constexpr float kBf16CondLimit = 256.0f;
+// The same decision at every replacement: the inner recursion claimed |r|^2
+// down by delta^2 since the last one, the true FP64 residual is down by about
+// (delta + u kappa)^2; a true ratio above kBf16Lag delta^2 means the BF16
+// rounding term dominates, and the cycles to come will crawl.
+constexpr double kBf16Lag = 10.0;
+__device__ __forceinline__ bool bf16_condition_ok(float ratio, int32_t k) {
+    if (!(ratio < 1.0f)) return false;   // no contraction at all (or NaN)
+    const float rho = powf(ratio, 0.5f / static_cast<float>(k));
+    const float s = (1.0f + rho) / (1.0f - rho);
+    return s * s <= kBf16CondLimit;
+}
+
 // ---------------------------------------------------------------------------
 // Cooperative grid solve (cg_coop.cu): the whole PCG loop of at most
 // kCoopMaxInst instances in one launch of one kCoopThreads-thread CTA per SM

@@ -419,22 +419,11 @@ cmcg_status launch_mixed_t(const MixArgs<MI, MO>& m, int nmax, size_t smem, int 
     return CMCG_OK;
 }
 
-template <typename MI, typename MO>
-cmcg_status launch_mixed_fast(const MixArgs<MI, MO>& m, int threads, int nmax, size_t smem, int nd, int grid,
-                              cudaStream_t stream) {
-    if (threads == 256) return launch_mixed_t<MI, MO, 256>(m, nmax, smem, nd, grid, stream);
-    if (threads == 512) return launch_mixed_t<MI, MO, 512>(m, nmax, smem, nd, grid, stream);
-    if (threads == kSmemThreads) return launch_mixed_t<MI, MO, kSmemThreads>(m, nmax, smem, nd, grid, stream);
-    return fail(CMCG_ERR_INVALID_ARGUMENT, "unsupported CTA size");
-}
-
-template cmcg_status launch_mixed_fast<float, float>(const MixArgs<float, float>&, int, int, size_t, int, int,
-                                                     cudaStream_t);
-template cmcg_status launch_mixed_fast<float, double>(const MixArgs<float, double>&, int, int, size_t, int, int,
-                                                      cudaStream_t);
-template cmcg_status launch_mixed_fast<__nv_bfloat16, float>(const MixArgs<__nv_bfloat16, float>&, int, int, size_t,
-                                                             int, int, cudaStream_t);
-template cmcg_status launch_mixed_fast<__nv_bfloat16, double>(const MixArgs<__nv_bfloat16, double>&, int, int, size_t,
-                                                              int, int, cudaStream_t);
+// One CTA size and inner value type per translation unit (the kernels take
+// minutes to compile; build.py compiles this file once per combination).
+template cmcg_status launch_mixed_t<CMCG_MIXED_MI, float, CMCG_MIXED_T>(const MixArgs<CMCG_MIXED_MI, float>&, int, size_t,
+                                                                        int, int, cudaStream_t);
+template cmcg_status launch_mixed_t<CMCG_MIXED_MI, double, CMCG_MIXED_T>(const MixArgs<CMCG_MIXED_MI, double>&, int,
+                                                                         size_t, int, int, cudaStream_t);
 
 }  // namespace cmcg

@@ -71,6 +71,7 @@ struct DiaPlan {
     int32_t* d_pos = nullptr;       // per CSR entry: its slot
     int64_t* d_sys_base = nullptr;  // n_sys
     int32_t* d_sys_off = nullptr;   // n_sys * kDiaMax
+    int32_t off0[kDiaMax] = {};     // the first system's offsets (host copy)
     int64_t plan_id = 0;            // changes when the systems change
 };
 

@@ -187,6 +187,7 @@ cmcg_status ensure_dia(cmcg_pattern p) {
         D.built = true;
         return st;
     }
+    std::copy(off.begin(), off.begin() + kDiaMax, D.off0);
     D.n_slots = slots;
     D.max_nd = nd_alloc;
     D.margin = margin;
