@@ -34,6 +34,7 @@
 #include "cg_compact.cuh"
 #include "cg_dev.cuh"
 #include "cg_smem.cuh"
+#include "cg_wide.cuh"
 #include "common.cuh"
 #include "cg_grid.cuh"
 #include "cg_plain.cuh"
@@ -1747,6 +1748,8 @@ struct cmcg_solver_s {
     bool cluster = true;
     // chip-resident solve of the grid path where it applies (CUMAT_CG_RESIDENT=0 disables)
     bool resident = true;
+    // one system of the cluster solve spread over all SMs (CUMAT_CG_WIDE=0 disables)
+    bool wide = true;
     void* res_ws = nullptr;   size_t res_ws_bytes = 0;
     // grid path: the product forms p_k (-1: by the batch's vector bytes against
     // L2, see fuse_p_update; 0 / 1: CUMAT_CG_FUSE)
@@ -2627,6 +2630,25 @@ cmcg_status run_cluster(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
     }
     if (nd != 5 && nd != 7) nd = 0;
     bool launched = false;
+    // one stencil system: spread over the SMs instead of one cluster, with the
+    // cluster's sums. us per iteration, here against the cluster (FP32 Poisson):
+    // 100^2 3.7 / 4.6, 200^2 4.0 / 6.3, 300^2 4.7 / 9.4; 3-D 7-point 27^3 4.4 / 5.5,
+    // 50^3 6.8 / 11.4; FP64 200^2 5.3 / 8.2, 40^3 7.9 / 10.0. FP64 with seven
+    // diagonals and at most two rows per thread stays on the cluster (27^3: 8.1 / 7.2).
+    if (FMT == CMCG_CSR && s->wide && n_inst == 1 && nd != 0 && !(sizeof(VT) == 8 && nd == 7 && lg < 12)) {
+        CMCG_TRY(ensure_buffer(&s->res_ws, &s->res_ws_bytes, wide_ws_bytes(c.rows, sizeof(VT))));
+        // (running until the launch says otherwise, as in run_coop)
+        CMCG_CUDA(cudaMemsetAsync(s->st.status, 0xFF, sizeof(int32_t), ctx->stream));
+        CMCG_CUDA(cudaMemsetAsync(s->st.rr, 0, sizeof(double), ctx->stream));
+        CMCG_CUDA(cudaMemsetAsync(s->st.bb, 0, sizeof(double), ctx->stream));
+        CMCG_TRY((wide_cg_launch<VT, MT>(c, lg, ctas, nd, ctx->sm_count, s->res_ws, ctx->d_err, ctx->stream, &launched)));
+        if (launched) {
+            if (log_on(2)) log_msg(2, "solve spread over all SMs: %d rows, %d rows per thread", c.rows, 1 << (lg - 10));
+            count_launch();
+            *done = true;
+            return CMCG_OK;
+        }
+    }
     CMCG_TRY((cluster_cg_launch<VT, MT, FMT>(c, n_inst, ctas, lg, nd, n_inst, ctx->stream, &launched)));
     if (!launched) {
         if (log_on(1))
@@ -3213,6 +3235,7 @@ cmcg_status cmcg_cg_create(cmcg_matrix A, int32_t precond, cmcg_solver* out) {
     if (const char* e = std::getenv("CUMAT_CG_SMALL")) s->mix_small = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_COOP")) s->coop = std::max(0, std::min(2, std::atoi(e)));
     if (const char* e = std::getenv("CUMAT_CG_CLUSTER")) s->cluster = std::atoi(e) != 0;
+    if (const char* e = std::getenv("CUMAT_CG_WIDE")) s->wide = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_RESIDENT")) s->resident = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_FUSE")) s->fuse_p = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_GRAPH")) s->graph_loop = std::atoi(e) != 0;

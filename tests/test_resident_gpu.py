@@ -1,6 +1,8 @@
-"""The chip-resident loop (cg_resident.cu) against the graph loop, whose order of
-additions it keeps: solutions, iteration counts and statuses are compared bit
-for bit; the graph loop is held to the oracle elsewhere."""
+"""Chip-resident forms of single-system solves against the paths whose sums they
+reproduce: the resident loop (cg_resident.cu) against the graph loop, the solve
+spread over all SMs (cg_wide.cu) against the cluster solve. Both keep the other
+path's order of additions, so solutions, iteration counts and statuses are
+compared bit for bit; the other paths are held to the oracle elsewhere."""
 import numpy as np
 import pytest
 import torch
@@ -161,7 +163,59 @@ def test_resident_statuses(cuda, monkeypatch):
         assert np.array_equal(out[0][0], out[1][0], equal_nan=True)
 
 
-@pytest.mark.parametrize("side,path", [(400, 2)])
+# the sizes at which a thread owns 1, 2, 4 and 8 rows; a last unit of one row;
+# fewer units than SMs and a last cluster CTA that is nearly empty
+WIDE = [("2d", 65), ("2d", 90), ("fv", 128), ("2d", 129), ("fv", 181), ("2d", 200), ("2d", 257), ("fv", 300),
+        ("2d", 362), ("3d", 17), ("3d", 25), ("3d", 40), ("3d", 50), ("band", (4097, (1, 2))),
+        ("band", (16385, (3, 7))), ("band", (131072, (1, 4099))), ("band", (32801, (1, 33, 1024)))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("kind,size", WIDE)
+def test_wide_equals_cluster(cuda, monkeypatch, kind, size, dtype):
+    m = cm()
+    row_ptr, col, val, b = _system(kind, size)
+    n = b.size
+    np_dt = np.float32 if dtype == torch.float32 else np.float64
+    A = m.SparseMatrix(m.SparsityPattern.csr(n, n, row_ptr, col), dtype=dtype).setData(val.astype(np_dt))
+    bt = torch.from_numpy(b.astype(np_dt)).to(cuda)
+    guess = torch.from_numpy(P.uniform(9, n).astype(np_dt)).to(cuda)
+    for precond in (True, False):
+        for g in (None, guess):
+            out = []
+            for env in ({}, {"CUMAT_CG_WIDE": "0", "CUMAT_CG_RESIDENT": "0"}):
+                cg = _solver(monkeypatch, A, env, precond).setTolerance(1e-6).setMaxIterations(200)
+                x = cg.solveWithGuess(bt, g).cpu().numpy()
+                out.append((x, cg.system_stats(), cg.error()))
+            assert out[0][1]["iterations"][0] == out[1][1]["iterations"][0]
+            assert out[0][1]["status"][0] == out[1][1]["status"][0]
+            if dtype == torch.float32 or n <= 65536:   # (larger FP64 systems: the graph and resident loops)
+                assert np.array_equal(out[0][0], out[1][0])
+                assert out[0][2] == out[1][2]
+    assert m.Context.current().device_errors() == 0
+
+
+def test_wide_statuses(cuda, monkeypatch):
+    m = cm()
+    row_ptr, col, val, b = _system("2d", 100)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    A, Neg = m.SparseMatrix(p).setData(val), m.SparseMatrix(p).setData(-val)
+    bt = torch.from_numpy(b).to(cuda)
+    bad = bt.clone()
+    bad[n // 3] = float("nan")
+    for M, rhs, limit in ((A, bt, 3), (A, bt, 0), (A, torch.zeros_like(bt), -1), (Neg, bt, -1), (A, bad, -1)):
+        out = []
+        for env in ({}, {"CUMAT_CG_WIDE": "0"}):
+            cg = _solver(monkeypatch, M, env, True).setTolerance(1e-6).setMaxIterations(limit)
+            x = cg.solve(rhs).cpu().numpy()
+            st = cg.system_stats()
+            out.append((x, int(st["iterations"][0]), int(st["status"][0])))
+        assert out[0][1:] == out[1][1:]
+        assert np.array_equal(out[0][0], out[1][0], equal_nan=True)
+
+
+@pytest.mark.parametrize("side,path", [(100, 0), (400, 2)])
 def test_tagged_word_waits_run_out(cuda, monkeypatch, side, path):
     # the readers wait for a tag that is never written: every poll runs out, the
     # device error bit is set, nothing is reported converged, and the context works
