@@ -38,7 +38,7 @@ CU_SOURCES = ["runtime.cu", "spmv.cu", "sell.cu", "sparse_ops.cu", "reduce.cu", 
               "lincomb.cu"]
 HEADERS = ["common.cuh", "objects.h", "spmv_dev.cuh", "cg_dev.cuh", "tma.cuh", "cg_smem.cuh", "cg_grid.cuh",
            "grid_sync.cuh", "cg_compact.cuh", "cg_plain.cuh", "cg_cluster.cuh",
-           "cg_resident.cuh", "cg_wide.cuh", "tagged.cuh"]
+           "cg_resident.cuh", "cg_wide.cuh", "tagged.cuh", "cg_onchip.cuh", "cg_onchip_dev.cuh"]
 
 
 def _stale(target: Path, deps: list[Path]) -> bool:
@@ -77,6 +77,7 @@ def build_cuda(verbose: bool = False, ptxas_info: bool = False) -> Path:
     objs = []
     units = [("cg_mixed.cu", f"cg_mixed.{t}.{mi}", [f"-DCMCG_MIXED_T={t}", f"-DCMCG_MIXED_MI={mi}"])
              for t, mi in MIXED_UNITS]   # (the slowest first)
+    units += [("cg_onchip.cu", "cg_onchip.f32", []), ("cg_onchip.cu", "cg_onchip.f64", ["-DCMCG_ONCHIP_FP64"])]
     units += [(src, src, []) for src in CU_SOURCES]
     for src, name, defs in units:
         s = CSRC / src

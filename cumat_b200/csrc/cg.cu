@@ -37,6 +37,7 @@
 #include "cg_wide.cuh"
 #include "common.cuh"
 #include "cg_grid.cuh"
+#include "cg_onchip.cuh"
 #include "cg_plain.cuh"
 #include "cg_resident.cuh"
 #include "objects.h"
@@ -1030,19 +1031,6 @@ __device__ __forceinline__ const MT* dia_system(const DiaArgs<MT>& d, int b, int
     return d.vals + (d.mb == 1 ? 0 : static_cast<int64_t>(b) * d.vstride) + __ldg(d.base + s);
 }
 
-// Values of a CSR matrix in the pattern's diagonal layout, unscaled:
-// dst[b][pos[k]] = vals[b][k] (thread per entry; other slots stay zero).
-template <typename MT>
-__global__ void k_dia_gather(const int32_t* __restrict__ pos, int64_t nnz, const MT* __restrict__ vals, int64_t vstride,
-                             int32_t mb, MT* __restrict__ dst, int64_t dstride) {
-    const int64_t items = nnz * mb;
-    for (int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; it < items;
-         it += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t b = it / nnz, k = it - b * nnz;
-        dst[b * dstride + pos[k]] = vals[b * vstride + k];
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Grid path kernels
 // ---------------------------------------------------------------------------
@@ -1724,6 +1712,8 @@ MatArgs<MT> mat_args(cmcg_matrix A) {
 // Solver object
 // ---------------------------------------------------------------------------
 
+constexpr int kAuxStreams = kOnchipForms64 - 1;   // launches of a batched solve beside the one on the caller's stream (six forms at most)
+
 struct cmcg_solver_s {
     cmcg_matrix A = nullptr;
     int32_t precond = CMCG_PRECOND_JACOBI;
@@ -1736,8 +1726,11 @@ struct cmcg_solver_s {
     // (CUMAT_CG_SMALL=0 keeps every system on 1024-thread CTAs)
     int32_t mix_split = 0, mix_split2 = 0;   // and >= mix_split2 on 256-thread CTAs
     bool mix_small = true;
-    cudaStream_t aux_stream[2] = {nullptr, nullptr};
-    cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
+    cudaStream_t aux_stream[kAuxStreams] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[kAuxStreams] = {};
+    std::vector<int32_t> order_rows;   // rows of the systems in size order (host copy of d_order's)
+    // on-chip batched kernels where they apply (CUMAT_CG_ONCHIP=0 disables)
+    bool onchip = true;
     bool use_smem = true;     // shared-memory-resident kernels where the systems fit
     bool inner_solve = false; // set while the solver runs the inner solves of a refinement
     bool fast_kernels = true; // compact-layout kernels where available (CUMAT_CG_FAST=0 disables)
@@ -1793,21 +1786,13 @@ struct cmcg_solver_s {
     void* mix_vals = nullptr;
     int64_t mix_stride = 0;
     double* mix_s = nullptr;
-    int64_t mix_version = -1, mix_plan_id = -1;
-    int32_t mix_dtype = -1;
+    int64_t mix_version = -1, mix_plan_id = -1, scale_version = -1;
     // the same scaled values in the pattern's diagonal layout, when it has one
     bool dia_kernels = true;  // CUMAT_CG_DIA=0 keeps the sliced layout
     void* dia_vals = nullptr;      // diagonal-layout values, then the unit-diagonal flags
     int32_t* dia_unit = nullptr;   // inside dia_vals
-    // the matrix's own (unscaled) values in the diagonal layout, for the plain
-    // grid-path product
-    void* dia_plain = nullptr;
-    int64_t dia_plain_stride = 0;
-    int64_t dia_plain_version = -1, dia_plain_plan_id = -1;
-    int32_t dia_plain_dtype = -1;
     int64_t dia_stride = 0;
     int64_t dia_version = -1, dia_plan_id = -1;
-    int32_t dia_dtype = -1;
     InstState st{};
     int32_t st_inst = 0;
     // graph cache of the grid path
@@ -1863,8 +1848,10 @@ cmcg_status build_plan(cmcg_solver s) {
     s->max_sys_rows = maxr;
     // last position of the size order with a system above kMixSmallRows rows
     s->mix_split = s->mix_split2 = 0;
+    s->order_rows.resize(n_sys);
     for (int32_t i = 0; i < n_sys; ++i) {
         const int64_t r = ro[order[i] + 1] - ro[order[i]];
+        s->order_rows[i] = static_cast<int32_t>(r);
         if (r > kMixSmallRows) s->mix_split = i + 1;
         if (r > kMixTinyRows) s->mix_split2 = i + 1;
     }
@@ -2077,21 +2064,21 @@ inline int smem_rows(int32_t max_rows) { return (max_rows + 3) / 4 * 4; }
 constexpr size_t kMixSmallSmemLimit = 104 * 1024;
 constexpr size_t kMixTinySmemLimit = 50 * 1024;
 
-// Streams of the highest and the next priority, and fork / join events, for
-// running the CTA tiers of the mixed kernel side by side (created on first use).
-// The five handles are created into locals and kept only when every creation
+// Streams of descending priority (from the highest) and fork / join events, for
+// running the CTA tiers of a batched solve side by side (created on first use).
+// The handles are created into locals and kept only when every creation
 // succeeded (a partial set is destroyed), so a failure leaves the solver
 // without any and the next call tries again.
 cmcg_status ensure_aux_stream(cmcg_solver s) {
-    if (s->aux_stream[0] && s->aux_stream[1] && s->ev_fork && s->ev_join[0] && s->ev_join[1]) return CMCG_OK;
+    if (s->ev_fork) return CMCG_OK;
     int least = 0, greatest = 0;
     CMCG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    cudaStream_t st[2] = {nullptr, nullptr};
-    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    cudaError_t e = cudaStreamCreateWithPriority(&st[0], cudaStreamNonBlocking, greatest);
-    if (e == cudaSuccess)
-        e = cudaStreamCreateWithPriority(&st[1], cudaStreamNonBlocking, std::min(least, greatest + 1));
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+    cudaStream_t st[kAuxStreams] = {};
+    cudaEvent_t ev[kAuxStreams + 1] = {};
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < kAuxStreams && e == cudaSuccess; ++k)
+        e = cudaStreamCreateWithPriority(&st[k], cudaStreamNonBlocking, std::min(least, greatest + k));
+    for (int k = 0; k <= kAuxStreams && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
     if (e != cudaSuccess) {
         for (auto x : st)
             if (x) cudaStreamDestroy(x);
@@ -2100,11 +2087,34 @@ cmcg_status ensure_aux_stream(cmcg_solver s) {
         cudaGetLastError();
         return fail(CMCG_ERR_CUDA, std::string("creating the tier streams: ") + cudaGetErrorString(e));
     }
-    s->aux_stream[0] = st[0];
-    s->aux_stream[1] = st[1];
-    s->ev_fork = ev[0];
-    s->ev_join[0] = ev[1];
-    s->ev_join[1] = ev[2];
+    for (int k = 0; k < kAuxStreams; ++k) {
+        s->aux_stream[k] = st[k];
+        s->ev_join[k] = ev[k];
+    }
+    s->ev_fork = ev[kAuxStreams];
+    return CMCG_OK;
+}
+
+// Launches `launch(j, stream)` for the nt tiers j side by side: the last on the
+// caller's stream, the others on the priority streams, joined back at the end.
+template <typename F>
+cmcg_status fork_tiers(cmcg_solver s, int nt, F&& launch) {
+    cmcg_ctx ctx = s->A->pat->ctx;
+    if (nt > 1) {
+        CMCG_TRY(ensure_aux_stream(s));
+        CMCG_CUDA(cudaEventRecord(s->ev_fork, ctx->stream));
+    }
+    for (int j = 0; j < nt; ++j) {
+        cudaStream_t st = (j == nt - 1) ? ctx->stream : s->aux_stream[j];
+        if (j < nt - 1) CMCG_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
+        CMCG_TRY(launch(j, st));
+        CMCG_CHECK_LAUNCH();
+        count_launch();
+    }
+    for (int j = 0; j < nt - 1; ++j) {
+        CMCG_CUDA(cudaEventRecord(s->ev_join[j], s->aux_stream[j]));
+        CMCG_CUDA(cudaStreamWaitEvent(ctx->stream, s->ev_join[j], 0));
+    }
     return CMCG_OK;
 }
 
@@ -2133,48 +2143,68 @@ inline CompactArgs compact_args(cmcg_pattern p) {
 }
 
 template <typename MT>
+cmcg_status build_scale(cmcg_solver s) {
+    cmcg_matrix A = s->A;
+    cmcg_pattern p = A->pat;
+    cmcg_ctx ctx = p->ctx;
+    k_jacobi_scale<MT><<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(p->d_row_ptr, p->d_col, static_cast<const MT*>(A->d_vals),
+                                                                   A->stride, p->rows, A->batches,
+                                                                   s->precond == CMCG_PRECOND_JACOBI ? 1 : 0, s->mix_s);
+    count_launch();
+    CMCG_CHECK_LAUNCH();
+    return CMCG_OK;
+}
+
+// The scale s = 1/sqrt(a_ii) of the mixed solves, recomputed when the matrix
+// values changed.
+cmcg_status ensure_scale(cmcg_solver s) {
+    cmcg_matrix A = s->A;
+    if (s->mix_s && s->scale_version == A->version) return CMCG_OK;
+    if (!s->mix_s)
+        CMCG_TRY(dev_alloc(reinterpret_cast<void**>(&s->mix_s),
+                           static_cast<size_t>(A->pat->rows) * A->batches * sizeof(double)));
+    CMCG_TRY(A->dtype == CMCG_F32 ? build_scale<float>(s) : A->dtype == CMCG_BF16 ? build_scale<__nv_bfloat16>(s)
+                                                                                  : build_scale<double>(s));
+    s->scale_version = A->version;
+    return CMCG_OK;
+}
+
+template <typename MT>
 cmcg_status build_mix(cmcg_solver s) {
     cmcg_matrix A = s->A;
     cmcg_pattern p = A->pat;
     cmcg_ctx ctx = p->ctx;
     const SellPlan& S = p->sell;
-    const int blocks = ctx->sm_count * 8;
-    k_jacobi_scale<MT><<<blocks, 256, 0, ctx->stream>>>(p->d_row_ptr, p->d_col, static_cast<const MT*>(A->d_vals), A->stride,
-                                                      p->rows, A->batches, s->precond == CMCG_PRECOND_JACOBI ? 1 : 0, s->mix_s);
-    k_scale_sell<MT, MT><<<blocks, 256, 0, ctx->stream>>>(S.d_col, S.d_slice_off, S.d_slice_w, S.d_slice_row0, S.n_slices,
-                                                         static_cast<const MT*>(A->d_sell_vals), A->sell_stride, s->mix_s,
-                                                         p->rows, A->batches, static_cast<MT*>(s->mix_vals), s->mix_stride);
-    count_launch(2);
+    k_scale_sell<MT, MT><<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(
+        S.d_col, S.d_slice_off, S.d_slice_w, S.d_slice_row0, S.n_slices, static_cast<const MT*>(A->d_sell_vals),
+        A->sell_stride, s->mix_s, p->rows, A->batches, static_cast<MT*>(s->mix_vals), s->mix_stride);
+    count_launch();
     CMCG_CHECK_LAUNCH();
     return CMCG_OK;
 }
 
-// Jacobi-scaled inner values and the scale vector of the mixed solver's fast
-// path, rebuilt when the matrix values or the systems changed.
+// Jacobi-scaled inner values in the sliced layout and the scale vector of the
+// mixed solves, rebuilt when the matrix values or the systems changed.
 cmcg_status ensure_mix(cmcg_solver s) {
     cmcg_matrix A = s->A;
-    cmcg_pattern p = A->pat;
+    CMCG_TRY(ensure_scale(s));
     CMCG_TRY(ensure_sell_values(A));
-    const SellPlan& S = p->sell;
-    if (s->mix_vals && s->mix_version == A->version && s->mix_plan_id == S.plan_id && s->mix_dtype == A->dtype)
-        return CMCG_OK;
-    dev_free(s->mix_vals);
-    dev_free(s->mix_s);
-    s->mix_vals = nullptr;
-    s->mix_s = nullptr;
-    s->mix_stride = A->sell_stride;
-    CMCG_TRY(dev_alloc(&s->mix_vals, static_cast<size_t>(s->mix_stride) * A->batches * dtype_size(A->dtype)));
-    CMCG_TRY(dev_alloc(reinterpret_cast<void**>(&s->mix_s), static_cast<size_t>(p->rows) * A->batches * sizeof(double)));
-    cmcg_status st = A->dtype == CMCG_F32 ? build_mix<float>(s) : A->dtype == CMCG_BF16 ? build_mix<__nv_bfloat16>(s)
-                                                                                        : build_mix<double>(s);
-    if (st != CMCG_OK) return st;
+    const SellPlan& S = A->pat->sell;
+    if (s->mix_vals && s->mix_version == A->version && s->mix_plan_id == S.plan_id) return CMCG_OK;
+    if (!s->mix_vals || s->mix_stride != A->sell_stride) {
+        dev_free(s->mix_vals);
+        s->mix_vals = nullptr;
+        CMCG_TRY(dev_alloc(&s->mix_vals, static_cast<size_t>(A->sell_stride) * A->batches * dtype_size(A->dtype)));
+        s->mix_stride = A->sell_stride;
+    }
+    CMCG_TRY(A->dtype == CMCG_F32 ? build_mix<float>(s) : A->dtype == CMCG_BF16 ? build_mix<__nv_bfloat16>(s)
+                                                                                : build_mix<double>(s));
     s->mix_version = A->version;
     s->mix_plan_id = S.plan_id;
-    s->mix_dtype = A->dtype;
     return CMCG_OK;
 }
 
-// Scaled inner values in the pattern's diagonal layout (after ensure_mix);
+// Scaled inner values in the pattern's diagonal layout (after ensure_scale);
 // false when the pattern has no diagonal plan.
 cmcg_status ensure_dia_vals(cmcg_solver s, bool* ok) {
     *ok = false;
@@ -2183,17 +2213,22 @@ cmcg_status ensure_dia_vals(cmcg_solver s, bool* ok) {
     CMCG_TRY(ensure_dia(p));
     const DiaPlan& D = p->dia;
     if (!D.ok) return CMCG_OK;
-    if (!(s->dia_vals && s->dia_version == A->version && s->dia_plan_id == D.plan_id && s->dia_dtype == A->dtype)) {
+    if (!(s->dia_vals && s->dia_version == A->version && s->dia_plan_id == D.plan_id)) {
         cmcg_ctx ctx = p->ctx;
-        dev_free(s->dia_vals);
-        s->dia_vals = nullptr;
-        s->dia_stride = (D.n_slots + 7) / 8 * 8 + 8;
-        // values, then the per-(batch, system) unit-diagonal flags
-        const size_t vbytes = (static_cast<size_t>(s->dia_stride) * A->batches * dtype_size(A->dtype) + 255) / 256 * 256;
-        const size_t bytes = vbytes + static_cast<size_t>(s->n_sys) * A->batches * sizeof(int32_t);
-        CMCG_TRY(dev_alloc(&s->dia_vals, bytes));
-        CMCG_CUDA(cudaMemsetAsync(s->dia_vals, 0, bytes, ctx->stream));
-        s->dia_unit = reinterpret_cast<int32_t*>(static_cast<char*>(s->dia_vals) + vbytes);
+        if (!s->dia_vals || s->dia_plan_id != D.plan_id) {
+            // (new values of the same plan overwrite the same slots: the others stay zero)
+            dev_free(s->dia_vals);
+            s->dia_vals = nullptr;
+            s->dia_stride = (D.n_slots + 7) / 8 * 8 + 8;
+            // values, then the per-(batch, system) unit-diagonal flags
+            const size_t vbytes =
+                (static_cast<size_t>(s->dia_stride) * A->batches * dtype_size(A->dtype) + 255) / 256 * 256;
+            const size_t bytes = vbytes + static_cast<size_t>(s->n_sys) * A->batches * sizeof(int32_t);
+            CMCG_TRY(dev_alloc(&s->dia_vals, bytes));
+            s->dia_plan_id = -1;
+            CMCG_CUDA(cudaMemsetAsync(s->dia_vals, 0, bytes, ctx->stream));
+            s->dia_unit = reinterpret_cast<int32_t*>(static_cast<char*>(s->dia_vals) + vbytes);
+        }
         const int blocks = ctx->sm_count * 8;
 #define CMCG_SCALE_DIA(MT)                                                                                              \
     k_scale_dia<MT><<<blocks, 256, 0, ctx->stream>>>(p->d_row_ptr, p->d_col, static_cast<const MT*>(A->d_vals), A->stride, \
@@ -2218,48 +2253,16 @@ cmcg_status ensure_dia_vals(cmcg_solver s, bool* ok) {
         CMCG_CHECK_LAUNCH();
         s->dia_version = A->version;
         s->dia_plan_id = D.plan_id;
-        s->dia_dtype = A->dtype;
     }
     *ok = true;
     return CMCG_OK;
 }
 
-// The matrix's values, unscaled, in the pattern's diagonal layout (rebuilt
-// when the values or the systems change); false when the pattern has no
-// diagonal plan or it is switched off.
+// The matrix's values, unscaled, in the pattern's diagonal layout; false when the
+// pattern has no diagonal plan or it is switched off.
 cmcg_status ensure_dia_plain(cmcg_solver s, bool* ok) {
     *ok = false;
-    cmcg_matrix A = s->A;
-    cmcg_pattern p = A->pat;
-    if (!s->dia_kernels || p->format != CMCG_CSR) return CMCG_OK;
-    CMCG_TRY(ensure_dia(p));
-    const DiaPlan& D = p->dia;
-    if (!D.ok) return CMCG_OK;
-    if (!(s->dia_plain && s->dia_plain_version == A->version && s->dia_plain_plan_id == D.plan_id &&
-          s->dia_plain_dtype == A->dtype)) {
-        cmcg_ctx ctx = p->ctx;
-        dev_free(s->dia_plain);
-        s->dia_plain = nullptr;
-        s->dia_plain_stride = (D.n_slots + 7) / 8 * 8 + 8;
-        const size_t bytes = static_cast<size_t>(s->dia_plain_stride) * A->batches * dtype_size(A->dtype);
-        CMCG_TRY(dev_alloc(&s->dia_plain, bytes));
-        CMCG_CUDA(cudaMemsetAsync(s->dia_plain, 0, bytes, ctx->stream));
-        const int blocks = ctx->sm_count * 8;
-#define CMCG_DIA_GATHER(MT)                                                                                   \
-    k_dia_gather<MT><<<blocks, 256, 0, ctx->stream>>>(D.d_pos, p->nnz, static_cast<const MT*>(A->d_vals), A->stride, \
-                                                      A->batches, static_cast<MT*>(s->dia_plain), s->dia_plain_stride)
-        if (A->dtype == CMCG_F32) CMCG_DIA_GATHER(float);
-        else if (A->dtype == CMCG_BF16) CMCG_DIA_GATHER(__nv_bfloat16);
-        else CMCG_DIA_GATHER(double);
-#undef CMCG_DIA_GATHER
-        count_launch();
-        CMCG_CHECK_LAUNCH();
-        s->dia_plain_version = A->version;
-        s->dia_plain_plan_id = D.plan_id;
-        s->dia_plain_dtype = A->dtype;
-    }
-    *ok = true;
-    return CMCG_OK;
+    return s->dia_kernels ? ensure_dia_values(s->A, ok) : CMCG_OK;
 }
 
 template <typename VT, typename MT, bool RX>
@@ -2307,8 +2310,8 @@ cmcg_status run_plain_dia(cmcg_solver s, SolveArgs<double, MT>& a, bool* done) {
     m.mb = s->A->batches;
     m.row_off = p->d_row_off;
     m.order = s->d_order;
-    m.vals = static_cast<const MT*>(s->dia_plain);
-    m.vstride = s->dia_plain_stride;
+    m.vals = static_cast<const MT*>(s->A->d_dia_vals);
+    m.vstride = s->A->dia_stride;
     m.base = D.d_sys_base;
     m.off = D.d_sys_off;
     m.margin = D.margin;
@@ -2332,28 +2335,163 @@ cmcg_status run_plain_dia(cmcg_solver s, SolveArgs<double, MT>& a, bool* done) {
     for (int t = 0; t < 3; ++t)
         if (lo[t + 1] > lo[t]) tiers[nt++] = t;
     CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 3 * sizeof(int32_t), ctx->stream));
-    if (nt > 1) {
-        CMCG_TRY(ensure_aux_stream(s));
-        CMCG_CUDA(cudaEventRecord(s->ev_fork, ctx->stream));
-    }
-    for (int j = 0; j < nt; ++j) {
+    CMCG_TRY(fork_tiers(s, nt, [&](int j, cudaStream_t st) -> cmcg_status {
         const int t = tiers[j];
-        cudaStream_t st = (j == nt - 1) ? ctx->stream : s->aux_stream[j];
-        if (j < nt - 1) CMCG_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
         PlainDiaArgs<MT> mt = m;
         mt.item_begin = lo[t];
         mt.item_end = lo[t + 1];
         mt.next = s->counters + t;
         const int grid = std::max(1, std::min(lo[t + 1] - lo[t], ctx->sm_count * (kSmemThreads / cta[t])));
-        CMCG_TRY(launch_plain_dia<MT>(mt, cta[t], nmax_t[t], sm_t[t], D.max_nd, grid, st));
-        CMCG_CHECK_LAUNCH();
-        count_launch();
-    }
-    for (int j = 0; j < nt - 1; ++j) {
-        CMCG_CUDA(cudaEventRecord(s->ev_join[j], s->aux_stream[j]));
-        CMCG_CUDA(cudaStreamWaitEvent(ctx->stream, s->ev_join[j], 0));
-    }
+        return launch_plain_dia<MT>(mt, cta[t], nmax_t[t], sm_t[t], D.max_nd, grid, st);
+    }));
     *done = true;
+    return CMCG_OK;
+}
+
+// Tiers of an on-chip batched solve: which systems (positions in the size
+// order) run on which launch form, and the form's dynamic shared memory.
+struct OnchipTier {
+    OnchipForm form;
+    int32_t lo, hi;
+    size_t smem;
+};
+
+// Dynamic shared memory of a CTA when per_sm of them share an SM: 228 KB, of
+// which every CTA takes 1 KB for the system and less than 2 KB of static arrays.
+inline size_t onchip_smem_limit(int per_sm) { return static_cast<size_t>(228 * 1024 / per_sm) - 3 * 1024; }
+// In the launches with FP32 vectors the systems share one CTA's memory, whose
+// static arrays are below 1 KB (plain) and 1.1 KB (mixed); a group of its threads
+// keeps its scratch in its part.
+inline size_t onchip_smem_limit32(int per_sm, bool mixed) {
+    const size_t scratch = mixed ? kOnchipMixScratch : kOnchipGroupScratch;
+    return static_cast<size_t>((227 * 1024 - (mixed ? 1280 : 1024)) / per_sm) - (per_sm > 1 ? scratch + 16 : 0);
+}
+
+// Splits the systems over the forms: each system takes the smallest form that
+// holds it (its shared memory and its rows), since more CTAs of fewer threads
+// share an SM there; with at most one instance per SM the forms that share an
+// SM are left out, which spreads the rows over more threads. The systems from
+// position `first` of the size order; empty when one fits no form.
+template <typename VT, int NF>
+std::vector<OnchipTier> onchip_tiers(cmcg_solver s, int32_t ob, const OnchipForm (&forms)[NF], int nd, size_t val_bytes,
+                                     bool mixed = false, int32_t first = 0) {
+    std::vector<OnchipTier> tiers;
+    const int margin = s->A->pat->dia.margin;
+    const bool few = static_cast<int64_t>(s->n_sys) * ob <= s->A->pat->ctx->sm_count;
+    const auto fits = [&](const OnchipForm& f, int rows) {
+        // (the mixed solve's order of sums, k_mixed_fast's, goes by size alone)
+        if (mixed) {
+            if (rows > kMixSmallRows || (f.threads == 512 ? rows <= kMixTinyRows : rows > kMixTinyRows)) return false;
+            if (few && f.threads == 128) return false;
+        } else if (few && f.per_sm > 1) {
+            return false;
+        }
+        const size_t b = onchip_smem<VT>(f, rows, nd, margin, val_bytes);
+        const bool whole = sizeof(VT) == 8 || (mixed && f.threads == 256);   // CTAs of this form share the SM, not a CTA's part
+        const size_t limit = whole ? onchip_smem_limit(f.per_sm) : onchip_smem_limit32(f.per_sm, mixed);
+        return b > 0 && b <= limit;
+    };
+    int32_t lo = first;
+    for (int f = 0; f < NF; ++f) {
+        // systems up to the last one that the next smaller forms do not hold
+        int32_t hi = s->n_sys;
+        if (f + 1 < NF) {
+            hi = lo;
+            for (int32_t i = s->n_sys; i > lo; --i) {
+                bool smaller = false;
+                for (int g = f + 1; g < NF && !smaller; ++g) smaller = fits(forms[g], s->order_rows[i - 1]);
+                if (!smaller) { hi = i; break; }
+            }
+        }
+        if (hi <= lo) continue;
+        const int rows = *std::max_element(s->order_rows.begin() + lo, s->order_rows.begin() + hi);
+        if (!fits(forms[f], rows)) return {};
+        tiers.push_back({forms[f], lo * ob, hi * ob, onchip_smem<VT>(forms[f], rows, nd, margin, val_bytes)});
+        lo = hi;
+    }
+    return tiers;
+}
+
+void log_tiers(const char* what, const std::vector<OnchipTier>& tiers) {
+    if (!log_on(2)) return;
+    for (const auto& t : tiers)
+        log_msg(2, "%s: %d instances on %d x %d threads, %zu bytes of shared memory", what, t.hi - t.lo, t.form.ctas,
+                t.form.threads, t.smem);
+}
+
+// Plain PCG of many stencil systems with their state on the chip
+// (cg_onchip.cu); *done = false where a system does not fit.
+template <typename VT, typename MT>
+cmcg_status run_onchip(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
+    *done = false;
+    if (!s->onchip || !s->fast_kernels || !s->use_smem || s->max_sys_rows > kSmemMaxRows) return CMCG_OK;
+    cmcg_pattern p = s->A->pat;
+    cmcg_ctx ctx = p->ctx;
+    bool dia = false;
+    CMCG_TRY(ensure_dia_plain(s, &dia));
+    if (!dia) return CMCG_OK;
+    const DiaPlan& D = p->dia;
+    std::vector<OnchipTier> tiers;
+    if constexpr (sizeof(VT) == 4) tiers = onchip_tiers<VT>(s, a.ob, kOnchip32, D.max_nd, sizeof(MT));
+    else tiers = onchip_tiers<VT>(s, a.ob, kOnchip64, D.max_nd, sizeof(MT));
+    if (tiers.empty()) return CMCG_OK;
+    OnchipArgs<VT, MT> m{};
+    m.rows = p->rows;
+    m.n_sys = s->n_sys;
+    m.ob = a.ob;
+    m.mb = s->A->batches;
+    m.row_off = p->d_row_off;
+    m.order = s->d_order;
+    m.vals = static_cast<const MT*>(s->A->d_dia_vals);
+    m.vstride = s->A->dia_stride;
+    m.base = D.d_sys_base;
+    m.off = D.d_sys_off;
+    m.margin = D.margin;
+    m.dinv = a.dinv;
+    m.dinv_b = a.dinv_b;
+    m.b = a.b;
+    m.b_b = a.b_b;
+    m.guess = a.guess;
+    m.g_b = a.g_b;
+    m.x = a.x;
+    m.tol = a.tol;
+    m.max_iter = a.max_iter;
+    m.abs_zero_test = a.abs_zero_test;
+    m.st = a.st;
+    CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 8 * sizeof(int32_t), ctx->stream));
+    if constexpr (sizeof(VT) == 4) {
+        // one launch: the CTAs go through the forms by themselves
+        OnchipWork w{};
+        size_t smem = 0;
+        int32_t at = 0;
+        for (int f = 0, j = 0; f < kOnchipForms32; ++f) {
+            w.t[f] = OnchipItems{s->counters + f, at, at};
+            if (j < static_cast<int>(tiers.size()) && tiers[j].form.threads == kOnchip32[f].threads &&
+                tiers[j].form.ctas == kOnchip32[f].ctas) {
+                w.t[f].lo = tiers[j].lo;
+                w.t[f].hi = at = tiers[j].hi;
+                const int k = kOnchip32[f].per_sm;
+                smem = std::max(smem, ((tiers[j].smem + 15) / 16 * 16 + (k > 1 ? kOnchipGroupScratch : 0)) * k);
+                ++j;
+            }
+        }
+        w.smem = static_cast<int32_t>((smem + 63) / 64 * 64);
+        CMCG_TRY((onchip_launch_all<MT>(m, w, D.max_nd, ctx->sm_count, ctx->stream, done)));
+        if (*done) count_launch();
+        CMCG_CHECK_LAUNCH();
+    } else {
+        bool all = true;
+        CMCG_TRY(fork_tiers(s, static_cast<int>(tiers.size()), [&](int j, cudaStream_t st) -> cmcg_status {
+            bool launched = false;
+            CMCG_TRY((onchip_launch<VT, MT>(m, OnchipItems{s->counters + j, tiers[j].lo, tiers[j].hi}, tiers[j].form,
+                                            tiers[j].smem, D.max_nd, ctx->sm_count, st, &launched)));
+            all = all && launched;
+            return CMCG_OK;
+        }));
+        // (a tier whose clusters the device cannot place: all systems again on the other kernels)
+        *done = all;
+    }
+    log_tiers("on-chip solve", tiers);
     return CMCG_OK;
 }
 
@@ -2450,7 +2588,7 @@ cmcg_status run_grid(cmcg_solver s, SolveArgs<VT, MT>& a) {
         if (dia) {
             const DiaPlan& D = s->A->pat->dia;
             nd = D.max_nd;
-            a.dia = DiaArgs<MT>{static_cast<const MT*>(s->dia_plain), s->dia_plain_stride, D.d_sys_base, D.d_sys_off,
+            a.dia = DiaArgs<MT>{static_cast<const MT*>(s->A->d_dia_vals), s->A->dia_stride, D.d_sys_base, D.d_sys_off,
                                 nullptr, s->A->batches};
         }
     }
@@ -2582,7 +2720,7 @@ cmcg_status run_resident(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
     CMCG_TRY(ensure_buffer(&s->res_ws, &s->res_ws_bytes, resident_ws_bytes(g, sizeof(VT))));
     a.part1 = static_cast<VT*>(s->part_ws);
     a.part2 = a.part1 + items;
-    a.dia = DiaArgs<MT>{static_cast<const MT*>(s->dia_plain), s->dia_plain_stride, D.d_sys_base, D.d_sys_off, nullptr,
+    a.dia = DiaArgs<MT>{static_cast<const MT*>(s->A->d_dia_vals), s->A->dia_stride, D.d_sys_base, D.d_sys_off, nullptr,
                         s->A->batches};
     CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 3 * sizeof(int32_t), st));
     k_grid_init<VT, MT, FMT><<<s->grid_ctas, kTile, 0, st>>>(a);
@@ -2624,7 +2762,7 @@ cmcg_status run_cluster(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
         if (dia) {
             const DiaPlan& D = s->A->pat->dia;
             nd = D.max_nd;
-            c.dia = DiaArgs<MT>{static_cast<const MT*>(s->dia_plain), s->dia_plain_stride, D.d_sys_base, D.d_sys_off,
+            c.dia = DiaArgs<MT>{static_cast<const MT*>(s->A->d_dia_vals), s->A->dia_stride, D.d_sys_base, D.d_sys_off,
                                 nullptr, s->A->batches};
         }
     }
@@ -2730,8 +2868,8 @@ cmcg_status solve_t(cmcg_solver s, const VT* b, int32_t b_b, const VT* guess, VT
     CMCG_TRY(ensure_state(s, n_inst));
     const void* dinv = nullptr;
     CMCG_TRY(get_dinv(s, DT<VT>::id, &dinv));
-    CMCG_TRY(ensure_sell_values(s->A));
-    const bool smem_ok = (FMT == CMCG_CSR && compact_ok(s)) || (sizeof(VT) == 4 && s->use_smem);
+    // (the sliced layout is built where a kernel reads it)
+    const bool smem_ok = s->use_smem && (sizeof(VT) == 4 || (FMT == CMCG_CSR && s->fast_kernels && s->max_sys_rows <= kSmemMaxRows));
     const int32_t path = choose_path(s, n_inst, smem_ok, /*cluster_ok=*/true);
     if (log_on(2))
         log_msg(2, "solve: %d instances of up to %d rows, %s vectors, %s path", n_inst, s->max_sys_rows,
@@ -2745,8 +2883,16 @@ cmcg_status solve_t(cmcg_solver s, const VT* b, int32_t b_b, const VT* guess, VT
         VT* w = static_cast<VT*>(s->vec_ws);
         a.b = b; a.b_b = b_b; a.guess = guess; a.g_b = ob; a.x = x;
         a.r = w; a.p = w + p->rows * static_cast<size_t>(ob); a.q = a.p + p->rows * static_cast<size_t>(ob);
-        CMCG_TRY((run_persistent<VT, MT, FMT>(s, a)));
+        bool done = false;
+        if (FMT == CMCG_CSR) CMCG_TRY(run_onchip(s, a, &done));
+        if (!done) {
+            CMCG_TRY(ensure_sell_values(s->A));
+            a.m = mat_args<MT>(s->A);
+            CMCG_TRY((run_persistent<VT, MT, FMT>(s, a)));
+        }
     } else {
+        CMCG_TRY(ensure_sell_values(s->A));
+        a.m = mat_args<MT>(s->A);
         // the graph iterates on internal copies of x so that its arguments do not
         // depend on the caller's buffers
         CMCG_TRY(ensure_vec_ws(s, 5 * vbytes + 256));
@@ -2822,7 +2968,7 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
     a.max_inner = s->max_iter;
     a.max_outer = max_outer;
     a.st = s->st;
-    CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 3 * sizeof(int32_t), ctx->stream));
+    CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 8 * sizeof(int32_t), ctx->stream));
     if (s->refine_method == CMCG_REFINE_RELIABLE && FMT == CMCG_CSR && compact_ok(s)) {
         CMCG_TRY(ensure_mix(s));
         MixArgs<MI, MO> m{};
@@ -2894,31 +3040,18 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
         int tiers[3], nt = 0;
         for (int t = 0; t < 3; ++t)
             if (lo[t + 1] > lo[t]) tiers[nt++] = t;
-        if (nt > 1) {
-            CMCG_TRY(ensure_aux_stream(s));
-            CMCG_CUDA(cudaEventRecord(s->ev_fork, ctx->stream));
-        }
         if (log_on(2))
             log_msg(2, "refined solve: %d instances on %d CTA tier(s) [%d, %d, %d instances], %s layout", n_inst, nt,
                     lo[1] - lo[0], lo[2] - lo[1], lo[3] - lo[2], nd ? "diagonal" : "sliced");
-        for (int j = 0; j < nt; ++j) {
+        CMCG_TRY(fork_tiers(s, nt, [&](int j, cudaStream_t st) -> cmcg_status {
             const int t = tiers[j];
-            // the last (smallest) tier runs on the caller's stream
-            cudaStream_t st = (j == nt - 1) ? ctx->stream : s->aux_stream[j];
-            if (j < nt - 1) CMCG_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
             MixArgs<MI, MO> mt = m;
             mt.item_begin = lo[t];
             mt.item_end = lo[t + 1];
             mt.next = s->counters + t;
             const int grid = std::max(1, std::min(lo[t + 1] - lo[t], ctx->sm_count * (kSmemThreads / cta[t])));
-            CMCG_TRY((launch_mixed_fast<MI, MO>(mt, cta[t], nmax_t[t], sm_t[t], nd, grid, st)));
-            CMCG_CHECK_LAUNCH();
-            count_launch();
-        }
-        for (int j = 0; j < nt - 1; ++j) {
-            CMCG_CUDA(cudaEventRecord(s->ev_join[j], s->aux_stream[j]));
-            CMCG_CUDA(cudaStreamWaitEvent(ctx->stream, s->ev_join[j], 0));
-        }
+            return launch_mixed_fast<MI, MO>(mt, cta[t], nmax_t[t], sm_t[t], nd, grid, st);
+        }));
         s->last_inst = n_inst;
         s->last_refined = true;
         return CMCG_OK;
@@ -3235,6 +3368,7 @@ cmcg_status cmcg_cg_create(cmcg_matrix A, int32_t precond, cmcg_solver* out) {
     if (const char* e = std::getenv("CUMAT_CG_SMALL")) s->mix_small = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_COOP")) s->coop = std::max(0, std::min(2, std::atoi(e)));
     if (const char* e = std::getenv("CUMAT_CG_CLUSTER")) s->cluster = std::atoi(e) != 0;
+    if (const char* e = std::getenv("CUMAT_CG_ONCHIP")) s->onchip = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_WIDE")) s->wide = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_RESIDENT")) s->resident = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_FUSE")) s->fuse_p = std::atoi(e) != 0;
@@ -3273,7 +3407,7 @@ cmcg_status cmcg_cg_destroy(cmcg_solver s) {
                     static_cast<void*>(s->d_cseg_sys), static_cast<void*>(s->d_ccta_seg0),
                     static_cast<void*>(s->d_csys_seg0), s->dinv[0], s->dinv[1], s->vec_ws, s->ref_ws, s->part_ws, s->res_ws,
                     s->st_ws, static_cast<void*>(s->counters), s->mix_vals, static_cast<void*>(s->mix_s),
-                    s->dia_vals, s->dia_plain})
+                    s->dia_vals})
         dev_free(p);
     if (s->host_io) cudaFreeHost(s->host_io);
     dev_free(s->fb_x);

@@ -143,6 +143,12 @@ struct cmcg_matrix_s {
     int64_t sell_stride = 0;
     int64_t sell_version = -1;
     int64_t sell_plan_id = -1;
+    // values in the pattern's diagonal layout ([batch][dia_stride], slots without
+    // an entry zero), regathered when `version` or the plan changes
+    void* d_dia_vals = nullptr;
+    int64_t dia_stride = 0;
+    int64_t dia_version = -1;
+    int64_t dia_plan_id = -1;
     // values in the entry order of the pattern's transpose ([batch][t_stride]),
     // regathered when `version` changes (the transposed product)
     void* d_t_vals = nullptr;
@@ -170,6 +176,9 @@ void free_sell(SellPlan& s);
 // builds the pattern's diagonal plan (CSR; dia.ok tells whether it applies)
 cmcg_status ensure_dia(cmcg_pattern p);
 void free_dia(DiaPlan& d);
+// the matrix's values in the pattern's diagonal layout; *ok = false when the
+// pattern has no diagonal plan
+cmcg_status ensure_dia_values(cmcg_matrix m, bool* ok);
 // values between the caller's order and the internal CSR order of a pattern
 // with d_val_perm (sparse_ops.cu): to_internal gathers dst[b][k] =
 // src[b][perm[k]], otherwise dst[b][perm[k]] = src[b][k]; dtype of both

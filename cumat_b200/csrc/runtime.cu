@@ -241,6 +241,7 @@ void matrix_release(cmcg_matrix m) {
     cudaStreamSynchronize(m->pat->ctx->stream);
     dev_free(m->d_vals);
     dev_free(m->d_sell_vals);
+    dev_free(m->d_dia_vals);
     dev_free(m->d_t_vals);
     cmcg_pattern p = m->pat;
     delete m;

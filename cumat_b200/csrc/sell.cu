@@ -251,4 +251,57 @@ cmcg_status ensure_sell_values(cmcg_matrix m) {
     return CMCG_OK;
 }
 
+namespace {
+
+// Values of a CSR matrix in the pattern's diagonal layout, unscaled:
+// dst[b][pos[k]] = vals[b][k] (thread per entry; other slots stay zero).
+template <typename MT>
+__global__ void k_dia_gather(const int32_t* __restrict__ pos, int64_t nnz, const MT* __restrict__ vals, int64_t vstride,
+                             int32_t mb, MT* __restrict__ dst, int64_t dstride) {
+    const int64_t items = nnz * mb;
+    for (int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; it < items;
+         it += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t b = it / nnz, k = it - b * nnz;
+        dst[b * dstride + pos[k]] = vals[b * vstride + k];
+    }
+}
+
+}  // namespace
+
+cmcg_status ensure_dia_values(cmcg_matrix m, bool* ok) {
+    *ok = false;
+    cmcg_pattern p = m->pat;
+    if (p->format != CMCG_CSR) return CMCG_OK;
+    CMCG_TRY(ensure_dia(p));
+    const DiaPlan& D = p->dia;
+    if (!D.ok) return CMCG_OK;
+    *ok = true;
+    if (m->d_dia_vals && m->dia_version == m->version && m->dia_plan_id == D.plan_id) return CMCG_OK;
+    cmcg_ctx ctx = p->ctx;
+    const int64_t stride = (D.n_slots + 7) / 8 * 8 + 8;
+    if (!m->d_dia_vals || m->dia_plan_id != D.plan_id) {
+        // (new values of the same plan overwrite the same slots: the others stay zero)
+        dev_free(m->d_dia_vals);
+        m->d_dia_vals = nullptr;
+        const size_t bytes = static_cast<size_t>(stride) * m->batches * dtype_size(m->dtype);
+        CMCG_TRY(dev_alloc(&m->d_dia_vals, bytes));
+        m->dia_stride = stride;
+        m->dia_plan_id = -1;
+        CMCG_CUDA(cudaMemsetAsync(m->d_dia_vals, 0, bytes, ctx->stream));
+    }
+    const int blocks = ctx->sm_count * 8;
+#define CMCG_DIA_GATHER(MT)                                                                                        \
+    k_dia_gather<MT><<<blocks, 256, 0, ctx->stream>>>(D.d_pos, p->nnz, static_cast<const MT*>(m->d_vals), m->stride, \
+                                                      m->batches, static_cast<MT*>(m->d_dia_vals), m->dia_stride)
+    if (m->dtype == CMCG_F32) CMCG_DIA_GATHER(float);
+    else if (m->dtype == CMCG_BF16) CMCG_DIA_GATHER(__nv_bfloat16);
+    else CMCG_DIA_GATHER(double);
+#undef CMCG_DIA_GATHER
+    count_launch();
+    CMCG_CHECK_LAUNCH();
+    m->dia_version = m->version;
+    m->dia_plan_id = D.plan_id;
+    return CMCG_OK;
+}
+
 }  // namespace cmcg
