@@ -35,7 +35,7 @@ NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--ex
 MIXED_UNITS = [(t, mi) for t in (256, 512, 1024) for mi in ("float", "__nv_bfloat16")]
 CU_SOURCES = ["runtime.cu", "spmv.cu", "sell.cu", "sparse_ops.cu", "reduce.cu", "cg.cu", "cg_plain.cu",
               "cg_coop.cu", "cg_cluster.cu", "cg_resident.cu", "cg_wide.cu",
-              "lincomb.cu"]
+              "cg_onchip_mixed.cu", "lincomb.cu"]
 HEADERS = ["common.cuh", "objects.h", "spmv_dev.cuh", "cg_dev.cuh", "tma.cuh", "cg_smem.cuh", "cg_grid.cuh",
            "grid_sync.cuh", "cg_compact.cuh", "cg_plain.cuh", "cg_cluster.cuh",
            "cg_resident.cuh", "cg_wide.cuh", "tagged.cuh", "cg_onchip.cuh", "cg_onchip_dev.cuh"]

@@ -2934,6 +2934,91 @@ cmcg_status solve_vt(cmcg_solver s, const VT* b, int32_t b_b, const VT* g, VT* x
 
 // ---- refined solve ----------------------------------------------------------------
 
+// On-chip part of a mixed batched solve (cg_onchip_mixed.cu): the systems from
+// position `first` of the size order (all of at most 8192 rows), in up to two
+// launches.
+template <typename MI, typename MO>
+struct OnchipMixPlan {
+    OnchipMixArgs<MI, MO> m;
+    OnchipItems items[3] = {};   // 512-, 256-, 128-thread form
+    int smem = 0;                // of the launch of the first and last form
+    size_t smem256 = 0;
+    int launches = 0;            // 0: not applicable
+    std::vector<OnchipTier> tiers;
+    bool first() const { return smem > 0; }   // a launch of the 512- and 128-thread forms
+    cmcg_status launch(cmcg_solver s, int j, cudaStream_t st) const {
+        const int nd = s->A->pat->dia.max_nd, sms = s->A->pat->ctx->sm_count;
+        bool launched = false;
+        if (j == 0 && first()) CMCG_TRY((onchip_mixed_launch<MI, MO>(m, items[0], items[2], smem, nd, sms, st, &launched)));
+        else CMCG_TRY((onchip_mixed_launch256<MI, MO>(m, items[1], smem256, nd, sms, st, &launched)));
+        return launched ? CMCG_OK : fail(CMCG_ERR_INTERNAL, "on-chip refined solve: unsupported number of diagonals");
+    }
+};
+
+template <typename MI, typename MO>
+cmcg_status onchip_mix_plan(cmcg_solver s, cmcg_matrix Ao, const double* b, int32_t b_b, double* x, int32_t ob,
+                            double outer_tol, int32_t max_outer, OnchipMixPlan<MI, MO>* plan) {
+    cmcg_pattern p = s->A->pat;
+    const int32_t first = s->mix_split;
+    if (!s->onchip || !s->fast_kernels || !s->use_smem || !s->dia_kernels || !s->mix_small || first >= s->n_sys ||
+        s->refine_method != CMCG_REFINE_RELIABLE || s->max_sys_rows > kSmemMaxRows)
+        return CMCG_OK;
+    bool dia = false;
+    CMCG_TRY(ensure_dia(p));
+    const DiaPlan& D = p->dia;
+    if (!D.ok) return CMCG_OK;
+    // k_mixed_fast's tiers, whose order of sums this keeps, exist while a vector's
+    // halo fits beside its small tiers' vectors
+    const auto tier_smem = [&](int32_t cap) {
+        const int32_t r = (std::min(s->max_sys_rows, cap) + kDiaBlockRows - 1) / kDiaBlockRows * kDiaBlockRows;
+        return smem_bytes(r) + 2 * sizeof(float) * static_cast<size_t>(D.margin);
+    };
+    if (tier_smem(kMixSmallRows) > kMixSmallSmemLimit || tier_smem(kMixTinyRows) > kMixTinySmemLimit) return CMCG_OK;
+    plan->tiers = onchip_tiers<float>(s, ob, kOnchipMix, D.max_nd, sizeof(MI), /*mixed=*/true, first);
+    if (plan->tiers.empty()) return CMCG_OK;
+    CMCG_TRY(ensure_dia_values(Ao, &dia));
+    CMCG_TRY(ensure_scale(s));
+    CMCG_TRY(ensure_dia_vals(s, &dia));
+    OnchipMixArgs<MI, MO>& m = plan->m;
+    m = OnchipMixArgs<MI, MO>{};
+    m.rows = p->rows;
+    m.n_sys = s->n_sys;
+    m.ob = ob;
+    m.mb = s->A->batches;
+    m.row_off = p->d_row_off;
+    m.order = s->d_order;
+    m.vin = static_cast<const MI*>(s->dia_vals);
+    m.vin_stride = s->dia_stride;
+    m.vout = static_cast<const MO*>(Ao->d_dia_vals);
+    m.vout_stride = Ao->dia_stride;
+    m.unit = s->dia_unit;
+    m.base = D.d_sys_base;
+    m.off = D.d_sys_off;
+    m.margin = D.margin;
+    m.s = s->mix_s;
+    m.b = b;
+    m.b_b = b_b;
+    m.x = x;
+    m.outer_tol = outer_tol;
+    m.max_inner = s->max_iter;
+    m.max_updates = max_outer;
+    m.delta = refine_delta_for(s);
+    m.st = s->st;
+    size_t smem = 0;
+    for (int f = 0; f < 3; ++f) plan->items[f] = OnchipItems{s->counters + 4 + f, 0, 0};
+    for (const OnchipTier& t : plan->tiers) {
+        const int f = t.form.threads == 512 ? 0 : t.form.threads == 256 ? 1 : 2;
+        plan->items[f].lo = t.lo;
+        plan->items[f].hi = t.hi;
+        if (f == 0) smem = std::max(smem, t.smem);
+        else if (f == 1) plan->smem256 = t.smem;
+        else smem = std::max(smem, ((t.smem + 15) / 16 * 16 + kOnchipMixScratch) * t.form.per_sm);
+    }
+    plan->smem = static_cast<int>((smem + 63) / 64 * 64);
+    plan->launches = (smem > 0 ? 1 : 0) + (plan->smem256 > 0 ? 1 : 0);
+    return CMCG_OK;
+}
+
 template <typename MI, typename MO, int FMT>
 cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, int32_t b_b, double* x, int32_t ob,
                                double outer_tol, int32_t max_outer) {
@@ -2941,6 +3026,16 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
     cmcg_ctx ctx = p->ctx;
     const int32_t n_inst = ob * s->n_sys;
     CMCG_TRY(ensure_state(s, n_inst));
+    OnchipMixPlan<MI, MO> on;
+    if (FMT == CMCG_CSR) CMCG_TRY((onchip_mix_plan<MI, MO>(s, Ao, b, b_b, x, ob, outer_tol, max_outer, &on)));
+    if (on.launches > 0 && s->mix_split == 0) {
+        CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 8 * sizeof(int32_t), ctx->stream));
+        CMCG_TRY(fork_tiers(s, on.launches, [&](int j, cudaStream_t st) { return on.launch(s, j, st); }));
+        log_tiers("on-chip refined solve", on.tiers);
+        s->last_inst = n_inst;
+        s->last_refined = true;
+        return CMCG_OK;
+    }
     const void* dinv = nullptr;
     CMCG_TRY(get_dinv(s, CMCG_F32, &dinv));
     const size_t nv = static_cast<size_t>(p->rows) * ob;
@@ -3039,11 +3134,13 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
         }
         int tiers[3], nt = 0;
         for (int t = 0; t < 3; ++t)
-            if (lo[t + 1] > lo[t]) tiers[nt++] = t;
+            if (lo[t + 1] > lo[t] && (t == 0 || on.launches == 0)) tiers[nt++] = t;
         if (log_on(2))
-            log_msg(2, "refined solve: %d instances on %d CTA tier(s) [%d, %d, %d instances], %s layout", n_inst, nt,
-                    lo[1] - lo[0], lo[2] - lo[1], lo[3] - lo[2], nd ? "diagonal" : "sliced");
-        CMCG_TRY(fork_tiers(s, nt, [&](int j, cudaStream_t st) -> cmcg_status {
+            log_msg(2, "refined solve: %d instances on %d CTA tier(s) [%d, %d, %d instances], %s layout%s", n_inst,
+                    nt + on.launches, lo[1] - lo[0], lo[2] - lo[1], lo[3] - lo[2], nd ? "diagonal" : "sliced",
+                    on.launches ? ", the smaller ones on the chip" : "");
+        CMCG_TRY(fork_tiers(s, nt + on.launches, [&](int j, cudaStream_t st) -> cmcg_status {
+            if (j >= nt) return on.launch(s, j - nt, st);
             const int t = tiers[j];
             MixArgs<MI, MO> mt = m;
             mt.item_begin = lo[t];

@@ -1,6 +1,7 @@
-"""On-chip batched solves (cg_onchip.cu) against the kernels they stand in for.
-The plain FP32 solve keeps the sums of the 1024-thread kernel in every launch
-form: bit for bit. FP64 solves are compared by statuses, iteration counts and solutions, and
+"""On-chip batched solves (cg_onchip.cu, cg_onchip_mixed.cu) against the kernels
+they stand in for. The plain FP32 solve keeps the sums of the 1024-thread kernel
+in every launch form and the mixed solve those of its kernel's tiers: bit for
+bit. FP64 solves are compared by statuses, iteration counts and solutions, and
 with the oracle elsewhere."""
 import numpy as np
 import pytest
@@ -113,6 +114,46 @@ def test_fp64_against_persistent(cuda, monkeypatch, name, values):
     assert np.all(np.abs(out[0][1]["iterations"] - out[1][1]["iterations"]) <= 2)
     # both residuals below 1e-12 |b|; |A^-1| |b| / |x| of these systems is below 1e3
     assert np.linalg.norm(out[0][0] - out[1][0]) <= 2e-9 * np.linalg.norm(out[1][0])
+
+
+@pytest.mark.parametrize("inner,outer", [(torch.float32, None), (torch.float32, torch.float64),
+                                         (torch.bfloat16, torch.float32), (torch.bfloat16, torch.float64)])
+@pytest.mark.parametrize("name", sorted(BATCHES))
+def test_mixed_equals_persistent(cuda, monkeypatch, name, inner, outer):
+    m = cm()
+    dims, sides = BATCHES[name]
+    off, row_ptr, col, val, b = _packed(sides, dims, 9)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p, dtype=inner).setData(val)
+    Ao = m.SparseMatrix(p, dtype=outer).setData(val) if outer else None
+    bt = torch.from_numpy(b.astype(np.float64)).to(cuda)
+    monkeypatch.setenv("CUMAT_CG_BF16_FALLBACK", "0")
+    out = []
+    for onchip in (True, False):
+        def make():
+            cg = m.ConjugateGradient(A).set_path(1)
+            return cg.solve_refined(bt, outer=Ao, outer_tol=1e-11, max_outer=200).cpu().numpy(), cg.system_stats()
+        out.append(_solve(monkeypatch, onchip, make))
+    assert np.array_equal(out[0][0], out[1][0])
+    for k in ("iterations", "status", "outer", "error"):
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
+    if inner == torch.float32:
+        assert np.all(out[0][1]["status"] == 0)
+
+
+def test_mixed_iteration_limit_reports_the_true_residual(cuda):
+    m = cm()
+    p1 = P.fv2d_batch(1, 100, 100, 0.5, 4)
+    A = m.SparseMatrix(m.SparsityPattern.csr(p1.n, p1.n, p1.row_ptr, p1.col)).setData(p1.val)
+    b = p1.b.astype(np.float64)
+    cg = m.ConjugateGradient(A).setMaxIterations(20)
+    x = cg.solve_refined(torch.from_numpy(b).to(cuda), outer_tol=1e-10).cpu().numpy()
+    st = cg.system_stats()
+    assert st["status"][0] == 1 and st["iterations"][0] == 20
+    r = b - np.add.reduceat(p1.val.astype(np.float64) * x[p1.col], p1.row_ptr[:-1])
+    assert abs(np.linalg.norm(r) / np.linalg.norm(b) - cg.error()) <= 1e-12
 
 
 @pytest.mark.parametrize("offsets", [(1, 7000), (3, 4099)])
