@@ -916,7 +916,7 @@ cmcg_status launch_dot(cmcg_ctx ctx, int64_t n, const void* x, int32_t xb, const
 // first gather and reused for all value batches; each product is
 // (alpha * u) * v, the reference's order.
 template <typename VT>
-__global__ void __launch_bounds__(kSpmvThreads) k_sddmm_csr(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+__global__ void __launch_bounds__(kSpmvThreads) k_sddmm_csr_rows(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                                             int32_t rows, int32_t cols, int64_t vstride, VT alpha,
                                                             const VT* __restrict__ u, int32_t ub,
                                                             const VT* __restrict__ v, int32_t vb,
@@ -961,6 +961,74 @@ __global__ void __launch_bounds__(kSpmvThreads) k_sddmm_csr(const int32_t* __res
     }
 }
 
+// The same with a warp for 32 rows: it takes 32 consecutive rows and writes their
+// entries, which are contiguous, 32 at a time: one coalesced store and index load
+// per 32 entries. A lane finds its entry's row among the warp's 32 row starts by
+// a five-step search with shuffles. The entry's row and column serve kSddmmBatch
+// value batches; several groups of batches of the same rows run on different
+// warps where the rows alone would leave SMs idle. Each product is
+// (alpha * u) * v, the reference's order. For patterns of few rows and many
+// value batches, where thread per row fills few SMs and each thread walks all
+// batches: 256 batches of 16,384 rows, 81,408 entries, FP64: 72 us (272 us thread
+// per row), bound by the output's stores. One batch of 4096^2 rows FP32: 516 us
+// (the search's instructions) against 276 us thread per row.
+constexpr int kSddmmBatch = 8;
+
+template <typename VT>
+__global__ void __launch_bounds__(kSpmvThreads) k_sddmm_csr_warp(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                                            int32_t rows, int32_t cols, int64_t vstride, VT alpha,
+                                                            const VT* __restrict__ u, int32_t ub,
+                                                            const VT* __restrict__ v, int32_t vb,
+                                                            VT* __restrict__ out, int32_t ob) {
+    const int lane = threadIdx.x & 31;
+    const int64_t groups = (static_cast<int64_t>(rows) + 31) / 32;
+    const int64_t bgroups = (ob + kSddmmBatch - 1) / kSddmmBatch;
+    const int64_t nw = static_cast<int64_t>(gridDim.x) * (kSpmvThreads / 32);
+    for (int64_t it = static_cast<int64_t>(blockIdx.x) * (kSpmvThreads / 32) + (threadIdx.x >> 5); it < groups * bgroups;
+         it += nw) {
+        const int64_t bg = it / groups, r0 = (it - bg * groups) * 32;
+        const int nr = static_cast<int>(min(static_cast<int64_t>(32), rows - r0));
+        const int b0 = static_cast<int>(bg) * kSddmmBatch, nb = min(kSddmmBatch, ob - b0);
+        // start of the lane's row (lanes past the last row: the end)
+        const int start = __ldg(rp + r0 + min(lane, nr));
+        const int lo = __shfl_sync(FULL, start, 0), hi = __ldg(rp + r0 + nr);
+        constexpr int U = 2;   // entries of a lane in flight
+        for (int k0 = lo; k0 < hi; k0 += 32 * U) {
+            int k[U], c[U], r[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                k[q] = k0 + 32 * q + lane;
+                c[q] = k[q] < hi ? __ldg(ci + k[q]) : 0;
+                // last row that starts at or before k (an empty row starts where
+                // the next one does, so it is never the last)
+                int row = 0;
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1) {
+                    const int t = row + s;
+                    const int at = __shfl_sync(FULL, start, t);
+                    if (t < nr && at <= k[q]) row = t;
+                }
+                r[q] = row;
+            }
+            const int64_t rb = r0;
+            for (int b = b0; b < b0 + nb; ++b) {
+                const VT* uu = u + (ub == 1 ? 0 : static_cast<int64_t>(b) * rows) + rb;
+                const VT* vv = v + (vb == 1 ? 0 : static_cast<int64_t>(b) * cols);
+                VT* o = out + static_cast<int64_t>(b) * vstride;
+                VT a[U], g[U];
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    a[q] = k[q] < hi ? __ldg(uu + r[q]) : VT(0);
+                    g[q] = k[q] < hi ? __ldg(vv + c[q]) : VT(0);
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    if (k[q] < hi) o[k[q]] = (alpha * a[q]) * g[q];
+            }
+        }
+    }
+}
+
 template <typename VT>
 __global__ void k_sddmm_ell(const int32_t* __restrict__ idx, int32_t width, int32_t rows_pad, int32_t rows, int32_t cols,
                             int64_t vstride, VT alpha, const VT* __restrict__ u, int32_t ub, const VT* __restrict__ v,
@@ -987,12 +1055,24 @@ cmcg_status launch_sddmm(cmcg_matrix M, double alpha, const void* u, int32_t ub,
     cmcg_pattern p = M->pat;
     cmcg_ctx ctx = p->ctx;
     if (p->format == CMCG_CSR) {
-        // two rows per thread; 64 registers leave 4 CTAs per SM
+        // thread per row, two rows per thread (64 registers leave 4 CTAs per SM), or
+        // a warp per 32 rows and group of batches where that grid would not fill
+        // the GPU once and there are batches to spread (both measured above)
         const int64_t need = (static_cast<int64_t>(p->rows) + 2 * kSpmvThreads - 1) / (2 * kSpmvThreads);
-        const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, ctx->sm_count * 4)));
-        k_sddmm_csr<VT><<<blocks, kSpmvThreads, 0, ctx->stream>>>(p->d_row_ptr, p->d_col, p->rows, p->cols, p->nnz,
-                                                         static_cast<VT>(alpha), static_cast<const VT*>(u), ub,
-                                                         static_cast<const VT*>(v), vb, static_cast<VT*>(out), ob);
+        const int64_t most = static_cast<int64_t>(ctx->sm_count) * 4;
+        if (ob == 1 || need >= most) {
+            const int blocks = static_cast<int>(std::max<int64_t>(1, std::min(need, most)));
+            k_sddmm_csr_rows<VT><<<blocks, kSpmvThreads, 0, ctx->stream>>>(
+                p->d_row_ptr, p->d_col, p->rows, p->cols, p->nnz, static_cast<VT>(alpha), static_cast<const VT*>(u), ub,
+                static_cast<const VT*>(v), vb, static_cast<VT*>(out), ob);
+        } else {
+            const int64_t warps = (static_cast<int64_t>(p->rows) + 31) / 32 * ((ob + kSddmmBatch - 1) / kSddmmBatch);
+            const int blocks = static_cast<int>(std::max<int64_t>(
+                1, std::min<int64_t>((warps + kSpmvThreads / 32 - 1) / (kSpmvThreads / 32), 2 * most)));
+            k_sddmm_csr_warp<VT><<<blocks, kSpmvThreads, 0, ctx->stream>>>(
+                p->d_row_ptr, p->d_col, p->rows, p->cols, p->nnz, static_cast<VT>(alpha), static_cast<const VT*>(u), ub,
+                static_cast<const VT*>(v), vb, static_cast<VT*>(out), ob);
+        }
     } else {
         const int64_t n = p->nnz * ob;
         const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, ctx->sm_count * 8));
