@@ -250,78 +250,74 @@ void matrix_release(cmcg_matrix m) {
 
 namespace {
 
-template <typename S, typename D>
-__global__ void k_convert(const S* __restrict__ src, D* __restrict__ dst, int64_t n);
+// Element conversions of value uploads (to BF16: round to nearest even).
+template <typename S, typename D> __device__ __forceinline__ D conv(S v) { return static_cast<D>(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 conv<float, __nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 conv<double, __nv_bfloat16>(double v) { return __double2bfloat16(v); }
+template <> __device__ __forceinline__ float conv<__nv_bfloat16, float>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <> __device__ __forceinline__ double conv<__nv_bfloat16, double>(__nv_bfloat16 v) {
+    return static_cast<double>(__bfloat162float(v));
+}
 
-template <>
-__global__ void k_convert<float, float>(const float* __restrict__ s, float* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = s[i];
-}
-template <>
-__global__ void k_convert<double, float>(const double* __restrict__ s, float* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = (float)s[i];
-}
-template <>
-__global__ void k_convert<float, double>(const float* __restrict__ s, double* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = (double)s[i];
-}
-template <>
-__global__ void k_convert<double, double>(const double* __restrict__ s, double* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = s[i];
-}
-template <>
-__global__ void k_convert<float, __nv_bfloat16>(const float* __restrict__ s, __nv_bfloat16* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = __float2bfloat16_rn(s[i]);
-}
-template <>
-__global__ void k_convert<double, __nv_bfloat16>(const double* __restrict__ s, __nv_bfloat16* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = __double2bfloat16(s[i]);
-}
-template <>
-__global__ void k_convert<__nv_bfloat16, __nv_bfloat16>(const __nv_bfloat16* __restrict__ s, __nv_bfloat16* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = s[i];
-}
-template <>
-__global__ void k_convert<__nv_bfloat16, float>(const __nv_bfloat16* __restrict__ s, float* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = __bfloat162float(s[i]);
-}
-template <>
-__global__ void k_convert<__nv_bfloat16, double>(const __nv_bfloat16* __restrict__ s, double* __restrict__ d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = (double)__bfloat162float(s[i]);
+// `runs` runs of n elements, run r from src + r sstride to dst + r dstride
+template <typename S, typename D>
+__global__ void __launch_bounds__(256) k_convert(const S* __restrict__ src, D* __restrict__ dst, int64_t n, int64_t runs,
+                                                 int64_t sstride, int64_t dstride) {
+    for (int64_t r = blockIdx.y; r < runs; r += gridDim.y) {
+        const S* __restrict__ s = src + r * sstride;
+        D* __restrict__ d = dst + r * dstride;
+        for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+             i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+            d[i] = conv<S, D>(s[i]);
+    }
 }
 
 template <typename S, typename D>
-cmcg_status launch_convert(cmcg_ctx ctx, const void* src, void* dst, int64_t n) {
-    if (n == 0) return CMCG_OK;
+cmcg_status launch_convert(cmcg_ctx ctx, const void* src, void* dst, int64_t n, int64_t runs, int64_t sstride,
+                           int64_t dstride) {
+    if (n == 0 || runs == 0) return CMCG_OK;
+    if (sstride == n && dstride == n) {   // one contiguous run
+        n *= runs;
+        runs = 1;
+    }
     const int threads = 256;
-    const int64_t want = (n + threads - 1) / threads;
-    const int blocks = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(ctx->sm_count) * 16));
-    k_convert<S, D><<<blocks, threads, 0, ctx->stream>>>(static_cast<const S*>(src), static_cast<D*>(dst), n);
+    const int64_t most = static_cast<int64_t>(ctx->sm_count) * 16;
+    const int64_t gx = std::min<int64_t>((n + threads - 1) / threads, most);
+    const int64_t gy = std::min<int64_t>(runs, std::max<int64_t>(1, std::min<int64_t>(65535, 2 * most / gx)));
+    k_convert<S, D><<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), threads, 0, ctx->stream>>>(
+        static_cast<const S*>(src), static_cast<D*>(dst), n, runs, sstride, dstride);
     count_launch();
     CMCG_CHECK_LAUNCH();
     return CMCG_OK;
 }
 
 template <typename S>
-cmcg_status convert_from(cmcg_ctx ctx, int dst_dt, const void* src, void* dst, int64_t n) {
+cmcg_status convert_from(cmcg_ctx ctx, int dst_dt, const void* src, void* dst, int64_t n, int64_t runs, int64_t sstride,
+                         int64_t dstride) {
     switch (dst_dt) {
-        case CMCG_F32: return launch_convert<S, float>(ctx, src, dst, n);
-        case CMCG_F64: return launch_convert<S, double>(ctx, src, dst, n);
-        case CMCG_BF16: return launch_convert<S, __nv_bfloat16>(ctx, src, dst, n);
+        case CMCG_F32: return launch_convert<S, float>(ctx, src, dst, n, runs, sstride, dstride);
+        case CMCG_F64: return launch_convert<S, double>(ctx, src, dst, n, runs, sstride, dstride);
+        case CMCG_BF16: return launch_convert<S, __nv_bfloat16>(ctx, src, dst, n, runs, sstride, dstride);
     }
     return fail(CMCG_ERR_INVALID_ARGUMENT, "unknown destination dtype");
+}
+
+// Converts runs of n elements (run r at src + r sstride, dst + r dstride) in one launch.
+cmcg_status convert_runs(cmcg_ctx ctx, int src_dt, const void* src, int dst_dt, void* dst, int64_t n, int64_t runs,
+                         int64_t sstride, int64_t dstride) {
+    switch (src_dt) {
+        case CMCG_F32: return convert_from<float>(ctx, dst_dt, src, dst, n, runs, sstride, dstride);
+        case CMCG_F64: return convert_from<double>(ctx, dst_dt, src, dst, n, runs, sstride, dstride);
+        case CMCG_BF16: return convert_from<__nv_bfloat16>(ctx, dst_dt, src, dst, n, runs, sstride, dstride);
+    }
+    return fail(CMCG_ERR_INVALID_ARGUMENT, "unknown source dtype");
 }
 
 }  // namespace
 
 // Converts n elements between element types on the context stream.
 cmcg_status convert(cmcg_ctx ctx, int src_dt, const void* src, int dst_dt, void* dst, int64_t n) {
-    switch (src_dt) {
-        case CMCG_F32: return convert_from<float>(ctx, dst_dt, src, dst, n);
-        case CMCG_F64: return convert_from<double>(ctx, dst_dt, src, dst, n);
-        case CMCG_BF16: return convert_from<__nv_bfloat16>(ctx, dst_dt, src, dst, n);
-    }
-    return fail(CMCG_ERR_INVALID_ARGUMENT, "unknown source dtype");
+    return convert_runs(ctx, src_dt, src, dst_dt, dst, n, 1, n, n);
 }
 
 }  // namespace cmcg
@@ -659,7 +655,7 @@ cmcg_status cmcg_matrix_set_values(cmcg_matrix m, int32_t src_dtype, const void*
     CMCG_CUDA(cudaSetDevice(ctx->device));
     const size_t es = dtype_size(src_dtype);
     // stage the user's dense batch-major layout on the device, then convert into
-    // the padded internal layout batch by batch (and slot by slot for ELL)
+    // the padded internal layout
     const int64_t per_batch = p->nnz;
     const size_t total = static_cast<size_t>(per_batch) * m->batches * es;
     void* stage = nullptr;
@@ -684,17 +680,12 @@ cmcg_status cmcg_matrix_set_values(cmcg_matrix m, int32_t src_dtype, const void*
         m->version++;
         return st;
     }
-    for (int32_t b = 0; b < m->batches && st == CMCG_OK; ++b) {
-        const char* sb = static_cast<const char*>(src) + static_cast<size_t>(b) * per_batch * es;
-        char* db = static_cast<char*>(m->d_vals) + static_cast<size_t>(b) * m->stride * ed;
-        if (p->format == CMCG_CSR) {
-            st = convert(ctx, src_dtype, sb, m->dtype, db, per_batch);
-        } else {
-            for (int32_t j = 0; j < p->width && st == CMCG_OK; ++j)
-                st = convert(ctx, src_dtype, sb + static_cast<size_t>(j) * p->rows * es, m->dtype,
-                             db + static_cast<size_t>(j) * p->rows_pad * ed, p->rows);
-        }
-    }
+    // all batches (ELL: all slots of all batches) in one launch: 256 value sets of
+    // 81,408 entries took 256 launches and 1.3 ms of host time
+    if (p->format == CMCG_CSR) st = convert_runs(ctx, src_dtype, src, m->dtype, m->d_vals, per_batch, m->batches, per_batch, m->stride);
+    else
+        st = convert_runs(ctx, src_dtype, src, m->dtype, m->d_vals, p->rows, static_cast<int64_t>(p->width) * m->batches,
+                          p->rows, p->rows_pad);
     if (stage) {
         cudaStreamSynchronize(ctx->stream);
         dev_free(stage);
