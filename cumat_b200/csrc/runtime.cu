@@ -681,7 +681,7 @@ cmcg_status cmcg_matrix_set_values(cmcg_matrix m, int32_t src_dtype, const void*
         return st;
     }
     // all batches (ELL: all slots of all batches) in one launch: 256 value sets of
-    // 81,408 entries took 256 launches and 1.3 ms of host time
+    // 81,408 entries took 256 launches and 1060 us, here 79 us (the copy's traffic)
     if (p->format == CMCG_CSR) st = convert_runs(ctx, src_dtype, src, m->dtype, m->d_vals, per_batch, m->batches, per_batch, m->stride);
     else
         st = convert_runs(ctx, src_dtype, src, m->dtype, m->d_vals, p->rows, static_cast<int64_t>(p->width) * m->batches,

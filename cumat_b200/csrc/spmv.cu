@@ -990,11 +990,13 @@ __global__ void __launch_bounds__(kSpmvThreads) k_sddmm_csr_warp(const int32_t* 
         const int nr = static_cast<int>(min(static_cast<int64_t>(32), rows - r0));
         const int b0 = static_cast<int>(bg) * kSddmmBatch, nb = min(kSddmmBatch, ob - b0);
         // start of the lane's row (lanes past the last row: the end)
-        const int start = __ldg(rp + r0 + min(lane, nr));
-        const int lo = __shfl_sync(FULL, start, 0), hi = __ldg(rp + r0 + nr);
+        // (unsigned: an entry index past the end may exceed 2^31 - 1)
+        const unsigned start = static_cast<unsigned>(__ldg(rp + r0 + min(lane, nr)));
+        const unsigned lo = __shfl_sync(FULL, start, 0), hi = static_cast<unsigned>(__ldg(rp + r0 + nr));
         constexpr int U = 2;   // entries of a lane in flight
-        for (int k0 = lo; k0 < hi; k0 += 32 * U) {
-            int k[U], c[U], r[U];
+        for (unsigned k0 = lo; k0 < hi; k0 += 32 * U) {
+            unsigned k[U];
+            int c[U], r[U];
 #pragma unroll
             for (int q = 0; q < U; ++q) {
                 k[q] = k0 + 32 * q + lane;
@@ -1005,7 +1007,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_sddmm_csr_warp(const int32_t* 
 #pragma unroll
                 for (int s = 16; s > 0; s >>= 1) {
                     const int t = row + s;
-                    const int at = __shfl_sync(FULL, start, t);
+                    const unsigned at = __shfl_sync(FULL, start, t);
                     if (t < nr && at <= k[q]) row = t;
                 }
                 r[q] = row;
