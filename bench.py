@@ -397,10 +397,14 @@ DRAM_PER_MODEL_BYTE = 0.004229
 # iteration on a 5-point system in the diagonal block layout with the unit
 # middle diagonal: 4 value loads (16 B) and 5 p reads (20 B) in the product,
 # r read + write (8 B), p read + write and the x-increment read + write
-# (16 B) in the updates. Each FP64 residual replacement moves per row 5 FP32
+# (16 B) in the updates. k_onchip_mixed, which solves the systems of up to 8192
+# rows, keeps r, x and the row's own p in registers: 4 value loads, 4 p reads and
+# one p write. Each FP64 residual replacement moves per row 5 FP32
 # values, 5 16-bit columns and 5 FP64 x gathers (70 B), b (8 B) and the new
 # FP32 residual (4 B), and its fold x += s * xh (read x, xh, s, write x: 28 B).
 L1_BYTES_PER_ROW_ITER = 60
+L1_BYTES_PER_ROW_ITER_ONCHIP = 36
+ONCHIP_ROWS = 8192
 L1_BYTES_PER_ROW_REPLACEMENT = 110
 # Nominal L1 data-pipe width: 128 B per clock per SM (32 banks x 4 B).
 L1_BYTES_PER_CLK_SM = 128
@@ -408,7 +412,8 @@ L1_BYTES_PER_CLK_SM = 128
 
 def l1_model_bytes(bt, inner_iters, outer_steps):
     n = np.diff(bt.row_off).astype(np.float64)
-    return float(np.sum(n * (inner_iters * L1_BYTES_PER_ROW_ITER + outer_steps * L1_BYTES_PER_ROW_REPLACEMENT)))
+    per_iter = np.where(n <= ONCHIP_ROWS, L1_BYTES_PER_ROW_ITER_ONCHIP, L1_BYTES_PER_ROW_ITER)
+    return float(np.sum(n * (inner_iters * per_iter + outer_steps * L1_BYTES_PER_ROW_REPLACEMENT)))
 
 
 def _ev_time(torch, stream, fn, reps, warm=1):
@@ -711,9 +716,10 @@ def run_ours(args):
     assert np.all(st["status"] == 0), "some systems did not converge"
     assert float(st["error"].max()) < OUTER_TOL
     value = whole_job_rate(N_SYS, world, ms)
-    # roofline of the dominant (only) kernel, k_mixed_fast: bound by the L1 /
-    # shared-memory data pipe (vectors live in shared memory, the values of the
-    # systems in flight in L2); the streaming model is kept as model_speedup
+    # roofline of the solve's kernels, k_mixed_fast (systems above 8192 rows,
+    # three quarters of the time) and k_onchip_mixed: bound by the L1 / shared-
+    # memory data pipe (vectors live in shared memory or registers, the values of
+    # the systems in flight in L2 or shared memory); the streaming model is kept as model_speedup
     inner = st["iterations"].astype(np.float64)
     outer = st["outer"].astype(np.float64)
     alg = refined_bytes(bt, inner, outer)
@@ -828,16 +834,17 @@ def run_ours(args):
                        "l2": "inputs larger than L2 (FP32 CSR batch %.2f GB)" % ((bt.nnz * 8 + bt.n * 4) / 1e9)},
             "roofline": {"bound": "l1_pipe", "achieved": round(l1_achieved, 1), "peak": round(l1_peak, 1),
                          "unit": "GB/s", "frac": round(l1_achieved / l1_peak, 3), "traffic": round(traffic),
-                         "kernel": "k_mixed_fast",
+                         "kernel": "k_mixed_fast + k_onchip_mixed",
                          "peak_source": f"nominal 128 B/clk/SM x {sm_count} SMs x median sampled SM clock {sm_mhz} MHz",
                          "l1_bytes_per_launch": l1_bytes,
                          "dram_frac": round(traffic / (ms / 1e3) / 1e9 / hbm_peak, 4),
                          "dram_peak_gbs": hbm_peak, "dram_peak_source": peak_src,
                          "model_speedup": round(alg / (ms / 1e3) / 1e9 / hbm_peak, 3),
                          # l1tex__data_pipe_lsu_wavefronts pct of peak per CTA tier, from the
-                         # k_mixed_fast ncu capture of the first 512 systems (--profile-small)
-                         "ncu_l1_pipe_pct_by_tier": {"1024": 54.5, "512": 32.7, "256": 19.3},
-                         "note": "achieved = L1-pipe model bytes (60 B per row and inner iteration) / time; traffic = "
+                         # k_mixed_fast ncu capture of the first 512 systems (--profile-small);
+                         # the smaller systems now run in k_onchip_mixed
+                         "ncu_l1_pipe_pct_by_tier": {"1024": 54.5},
+                         "note": "achieved = L1-pipe model bytes (60 B per row and inner iteration, 36 B up to 8192 rows) / time; traffic = "
                                  "DRAM bytes per launch scaled from an ncu capture; model_speedup = HBM streaming "
                                  "model time / measured time"},
             "cpu_baseline": cpu,
@@ -1010,7 +1017,7 @@ def run_profile_case(case: str):
                 path: plain FP64 Jacobi-CG and the mixed FP32 / FP64 solve,
                 each capped at 20 inner iterations (k_grid_*, k_gmix_*)
     plain_dia   plain FP64 batched CG of the first 512 systems of the batch
-                to 1e-10 (k_plain_dia, three CTA tiers)
+                to 1e-10 (k_onchip, a launch per form)
     vectors     dot, squared norm, linear combination of 4 terms and the
                 sampled outer product on n = 64 Mi entries (k_dot, k_lincomb,
                 k_sddmm_csr on the 8192^2 Poisson pattern)

@@ -2369,8 +2369,12 @@ inline size_t onchip_smem_limit32(int per_sm, bool mixed) {
 
 // Splits the systems over the forms: each system takes the smallest form that
 // holds it (its shared memory and its rows), since more CTAs of fewer threads
-// share an SM there; with at most one instance per SM the forms that share an
-// SM are left out, which spreads the rows over more threads. The systems from
+// share an SM there (592 systems of 4096 rows, FP64: 2.7 ms two to an SM, 7.5 ms
+// for the next size, 4225 rows, one to an SM); with at most one instance per SM
+// the forms that share an SM are left out, which spreads the rows over more
+// threads. The fallback for systems no form holds is the kernel each form is
+// measured against: FP32 20 .. 128 rows square 1.4 .. 3.6x slower, FP64 1.1 ..
+// 6.4x, mixed up to 8192 rows 1.1 .. 1.9x. The systems from
 // position `first` of the size order; empty when one fits no form.
 template <typename VT, int NF>
 std::vector<OnchipTier> onchip_tiers(cmcg_solver s, int32_t ob, const OnchipForm (&forms)[NF], int nd, size_t val_bytes,

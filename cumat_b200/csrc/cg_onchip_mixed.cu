@@ -15,7 +15,7 @@
 // cluster of two CTAs (its three cluster barriers an iteration took 5,000 of
 // 11,000 cycles) and with 32 rows per thread and values from L2 (spills): 296
 // systems of 16,384 rows to 1e-10 8.7 ms there, 12.4 ms in the second form. Below:
-// 592 systems of 8100 rows 6.1 ms there, 4.1 here.
+// 592 systems of 8100 rows 6.2 ms there, 3.9 here.
 #include <type_traits>
 
 #include "cg_dev.cuh"
