@@ -38,7 +38,8 @@ CU_SOURCES = ["runtime.cu", "spmv.cu", "sell.cu", "sparse_ops.cu", "reduce.cu", 
               "cg_onchip_mixed.cu", "lincomb.cu"]
 HEADERS = ["common.cuh", "objects.h", "spmv_dev.cuh", "cg_dev.cuh", "tma.cuh", "cg_smem.cuh", "cg_grid.cuh",
            "grid_sync.cuh", "cg_compact.cuh", "cg_plain.cuh", "cg_cluster.cuh",
-           "cg_resident.cuh", "cg_wide.cuh", "tagged.cuh", "cg_onchip.cuh", "cg_onchip_dev.cuh"]
+           "cg_resident.cuh", "cg_wide.cuh", "tagged.cuh", "cg_onchip.cuh", "cg_onchip_dev.cuh",
+           "cg_onchip_tiers.h"]
 
 
 def _stale(target: Path, deps: list[Path]) -> bool:

@@ -1728,7 +1728,9 @@ struct cmcg_solver_s {
     bool mix_small = true;
     cudaStream_t aux_stream[kAuxStreams] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[kAuxStreams] = {};
-    std::vector<int32_t> order_rows;   // rows of the systems in size order (host copy of d_order's)
+    // host copies: the systems in size order (d_order), their rows, and the
+    // largest |offset| of each (filled from the diagonal plan on first use)
+    std::vector<int32_t> order, order_rows, order_reach;
     // on-chip batched kernels where they apply (CUMAT_CG_ONCHIP=0 disables)
     bool onchip = true;
     bool use_smem = true;     // shared-memory-resident kernels where the systems fit
@@ -1848,6 +1850,8 @@ cmcg_status build_plan(cmcg_solver s) {
     s->max_sys_rows = maxr;
     // last position of the size order with a system above kMixSmallRows rows
     s->mix_split = s->mix_split2 = 0;
+    s->order = order;
+    s->order_reach.clear();
     s->order_rows.resize(n_sys);
     for (int32_t i = 0; i < n_sys; ++i) {
         const int64_t r = ro[order[i] + 1] - ro[order[i]];
@@ -2348,72 +2352,15 @@ cmcg_status run_plain_dia(cmcg_solver s, SolveArgs<double, MT>& a, bool* done) {
     return CMCG_OK;
 }
 
-// Tiers of an on-chip batched solve: which systems (positions in the size
-// order) run on which launch form, and the form's dynamic shared memory.
-struct OnchipTier {
-    OnchipForm form;
-    int32_t lo, hi;
-    size_t smem;
-};
+static_assert(kOnchipMixRows == kMixSmallRows && kOnchipMixTinyRows == kMixTinyRows, "");
 
-// Dynamic shared memory of a CTA when per_sm of them share an SM: 228 KB, of
-// which every CTA takes 1 KB for the system and less than 2 KB of static arrays.
-inline size_t onchip_smem_limit(int per_sm) { return static_cast<size_t>(228 * 1024 / per_sm) - 3 * 1024; }
-// In the launches with FP32 vectors the systems share one CTA's memory, whose
-// static arrays are below 1 KB (plain) and 1.1 KB (mixed); a group of its threads
-// keeps its scratch in its part.
-inline size_t onchip_smem_limit32(int per_sm, bool mixed) {
-    const size_t scratch = mixed ? kOnchipMixScratch : kOnchipGroupScratch;
-    return static_cast<size_t>((227 * 1024 - (mixed ? 1280 : 1024)) / per_sm) - (per_sm > 1 ? scratch + 16 : 0);
-}
-
-// Splits the systems over the forms: each system takes the smallest form that
-// holds it (its shared memory and its rows), since more CTAs of fewer threads
-// share an SM there (592 systems of 4096 rows, FP64: 2.7 ms two to an SM, 7.5 ms
-// for the next size, 4225 rows, one to an SM); with at most one instance per SM
-// the forms that share an SM are left out, which spreads the rows over more
-// threads. The fallback for systems no form holds is the kernel each form is
-// measured against: FP32 20 .. 128 rows square 1.4 .. 3.6x slower, FP64 1.1 ..
-// 6.4x, mixed up to 8192 rows 1.1 .. 1.9x. The systems from
-// position `first` of the size order; empty when one fits no form.
-template <typename VT, int NF>
-std::vector<OnchipTier> onchip_tiers(cmcg_solver s, int32_t ob, const OnchipForm (&forms)[NF], int nd, size_t val_bytes,
-                                     bool mixed = false, int32_t first = 0) {
-    std::vector<OnchipTier> tiers;
-    const int margin = s->A->pat->dia.margin;
-    const bool few = static_cast<int64_t>(s->n_sys) * ob <= s->A->pat->ctx->sm_count;
-    const auto fits = [&](const OnchipForm& f, int rows) {
-        // (the mixed solve's order of sums, k_mixed_fast's, goes by size alone)
-        if (mixed) {
-            if (rows > kMixSmallRows || (f.threads == 512 ? rows <= kMixTinyRows : rows > kMixTinyRows)) return false;
-            if (few && f.threads == 128) return false;
-        } else if (few && f.per_sm > 1) {
-            return false;
-        }
-        const size_t b = onchip_smem<VT>(f, rows, nd, margin, val_bytes);
-        const bool whole = sizeof(VT) == 8 || (mixed && f.threads == 256);   // CTAs of this form share the SM, not a CTA's part
-        const size_t limit = whole ? onchip_smem_limit(f.per_sm) : onchip_smem_limit32(f.per_sm, mixed);
-        return b > 0 && b <= limit;
-    };
-    int32_t lo = first;
-    for (int f = 0; f < NF; ++f) {
-        // systems up to the last one that the next smaller forms do not hold
-        int32_t hi = s->n_sys;
-        if (f + 1 < NF) {
-            hi = lo;
-            for (int32_t i = s->n_sys; i > lo; --i) {
-                bool smaller = false;
-                for (int g = f + 1; g < NF && !smaller; ++g) smaller = fits(forms[g], s->order_rows[i - 1]);
-                if (!smaller) { hi = i; break; }
-            }
-        }
-        if (hi <= lo) continue;
-        const int rows = *std::max_element(s->order_rows.begin() + lo, s->order_rows.begin() + hi);
-        if (!fits(forms[f], rows)) return {};
-        tiers.push_back({forms[f], lo * ob, hi * ob, onchip_smem<VT>(forms[f], rows, nd, margin, val_bytes)});
-        lo = hi;
-    }
-    return tiers;
+// The solver's systems for the tier rule (after ensure_dia).
+OnchipBatch onchip_batch(cmcg_solver s, int32_t ob, size_t val_bytes, bool mixed = false, int32_t first = 0) {
+    const DiaPlan& D = s->A->pat->dia;
+    if (s->order_reach.empty())
+        for (int32_t i : s->order) s->order_reach.push_back(D.reach[i]);
+    return OnchipBatch{s->order_rows.data(), s->order_reach.data(), s->n_sys, first, ob, s->A->pat->ctx->sm_count,
+                       D.max_nd, D.margin, val_bytes, mixed};
 }
 
 void log_tiers(const char* what, const std::vector<OnchipTier>& tiers) {
@@ -2436,8 +2383,8 @@ cmcg_status run_onchip(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
     if (!dia) return CMCG_OK;
     const DiaPlan& D = p->dia;
     std::vector<OnchipTier> tiers;
-    if constexpr (sizeof(VT) == 4) tiers = onchip_tiers<VT>(s, a.ob, kOnchip32, D.max_nd, sizeof(MT));
-    else tiers = onchip_tiers<VT>(s, a.ob, kOnchip64, D.max_nd, sizeof(MT));
+    if constexpr (sizeof(VT) == 4) tiers = onchip_tiers<VT>(onchip_batch(s, a.ob, sizeof(MT)), kOnchip32);
+    else tiers = onchip_tiers<VT>(onchip_batch(s, a.ob, sizeof(MT)), kOnchip64);
     if (tiers.empty()) return CMCG_OK;
     OnchipArgs<VT, MT> m{};
     m.rows = p->rows;
@@ -2978,7 +2925,7 @@ cmcg_status onchip_mix_plan(cmcg_solver s, cmcg_matrix Ao, const double* b, int3
         return smem_bytes(r) + 2 * sizeof(float) * static_cast<size_t>(D.margin);
     };
     if (tier_smem(kMixSmallRows) > kMixSmallSmemLimit || tier_smem(kMixTinyRows) > kMixTinySmemLimit) return CMCG_OK;
-    plan->tiers = onchip_tiers<float>(s, ob, kOnchipMix, D.max_nd, sizeof(MI), /*mixed=*/true, first);
+    plan->tiers = onchip_tiers<float>(onchip_batch(s, ob, sizeof(MI), /*mixed=*/true, first), kOnchipMix);
     if (plan->tiers.empty()) return CMCG_OK;
     CMCG_TRY(ensure_dia_values(Ao, &dia));
     CMCG_TRY(ensure_scale(s));

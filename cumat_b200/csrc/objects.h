@@ -72,6 +72,7 @@ struct DiaPlan {
     int64_t* d_sys_base = nullptr;  // n_sys
     int32_t* d_sys_off = nullptr;   // n_sys * kDiaMax
     int32_t off0[kDiaMax] = {};     // the first system's offsets (host copy)
+    std::vector<int32_t> reach;     // per system: its largest |offset| (host)
     int64_t plan_id = 0;            // changes when the systems change
 };
 

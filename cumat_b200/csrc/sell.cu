@@ -131,7 +131,7 @@ cmcg_status ensure_dia(cmcg_pattern p) {
     const int64_t n_sys = static_cast<int64_t>(ro.size()) - 1;
     std::vector<int32_t> off(static_cast<size_t>(n_sys) * kDiaMax, 0);
     std::vector<int64_t> base(n_sys);
-    std::vector<int32_t> nd(n_sys);
+    std::vector<int32_t> nd(n_sys), reach(n_sys, 0);
     int64_t slots = 0;
     int32_t max_nd = 0, margin = 0;
     for (int64_t s = 0; s < n_sys; ++s) {
@@ -148,8 +148,9 @@ cmcg_status ensure_dia(cmcg_pattern p) {
         std::sort(o.begin(), o.end());
         for (size_t j = 0; j < o.size(); ++j) {
             off[static_cast<size_t>(s) * kDiaMax + j] = o[j];
-            margin = std::max(margin, std::abs(o[j]));
+            reach[s] = std::max(reach[s], std::abs(o[j]));
         }
+        margin = std::max(margin, reach[s]);
         nd[s] = static_cast<int32_t>(o.size());
         max_nd = std::max(max_nd, nd[s]);
     }
@@ -188,6 +189,7 @@ cmcg_status ensure_dia(cmcg_pattern p) {
         return st;
     }
     std::copy(off.begin(), off.begin() + kDiaMax, D.off0);
+    D.reach = std::move(reach);
     D.n_slots = slots;
     D.max_nd = nd_alloc;
     D.margin = margin;

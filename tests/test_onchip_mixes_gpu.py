@@ -1,0 +1,75 @@
+"""Batched solves whose systems differ in shape: squares, long grids and bands of
+one batch, for which the launch forms of cg_onchip.cu differ in their halos. The
+solutions are held to their residual, formed with NumPy in 64 bits: a solve that
+stops at |r| < tol |b| has a true residual within tol |b| plus the drift of the
+recursion, at most (iterations) (unit roundoff) (|A| |x| / |b|), below 1e3 * 1e-16 *
+1e3 for these systems in FP64."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from cumat_b200 import problems as P  # noqa: E402
+from test_resident_gpu import _banded  # noqa: E402
+
+
+def cm():
+    import cumat_b200
+    return cumat_b200
+
+
+def _pack(systems, seed):
+    """Packed systems (rows, offsets): row offsets, CSR arrays, right-hand side."""
+    parts = {}
+    out = []
+    for i, key in enumerate(systems):
+        if key not in parts:
+            parts[key] = _banded(*key, seed + i)
+        out.append(parts[key])
+    off = np.concatenate([[0], np.cumsum([k[0] for k in systems])]).astype(np.int64)
+    nz = np.concatenate([[0], np.cumsum([p[1].size for p in out])])
+    row_ptr = np.concatenate([p[0][:-1] + nz[i] for i, p in enumerate(out)] + [[nz[-1]]]).astype(np.int32)
+    col = np.concatenate([p[1] + off[i] for i, p in enumerate(out)]).astype(np.int32)
+    return off, row_ptr, col, np.concatenate([p[2] for p in out]), P.uniform(seed, int(off[-1]))
+
+
+def _residuals(off, row_ptr, col, val, b, x):
+    """|b - A x| / |b| per system, in 64 bits."""
+    r = b.astype(np.float64) - np.add.reduceat(val.astype(np.float64) * x.astype(np.float64)[col], row_ptr[:-1])
+    n2 = lambda v: np.sqrt(np.add.reduceat(v.astype(np.float64) ** 2, off[:-1]))  # noqa: E731
+    return n2(r) / n2(b)
+
+
+def _square(s):
+    return (s * s, (1, s))
+
+
+def _grid(w, h, d=0):
+    return (w * h * max(d, 1), (1, w, w * h) if d else (1, w))
+
+
+# systems of one batch that take different forms: a long grid whose halo spans more
+# than a CTA's rows, and small systems that the batch's halo keeps out of the
+# smallest forms; the last one is reached by FP32 values under FP64 vectors
+MIXES = {"long_grid": [_square(100)] * 10 + [_grid(2200, 2)] + [_square(58)] * 2,
+         "long_grid_3d": [(13000, (1, 100, 1300)), _grid(50, 70, 3), (9000, (1, 90, 900))],
+         "band": [_square(128)] * 10 + [(5000, (1, 3500))],
+         "band_alone": [(5000, (1, 2499)), (4100, (3, 2100)), (9000, (1, 3000)), (12000, (7, 3071))],
+         "wide": [_square(64)] * 150 + [_grid(3000, 3), _grid(1025, 15), _square(20)],
+         "small": [_grid(700, 2), _grid(2, 700), _square(31), (50, (1,)), (3, (2,))] * 40}
+
+
+@pytest.mark.parametrize("values", [torch.float64, torch.float32])
+@pytest.mark.parametrize("name", sorted(MIXES))
+def test_fp64_mixed_shapes(cuda, name, values):
+    m = cm()
+    off, row_ptr, col, val, b = _pack(MIXES[name], 11)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p, dtype=values).setData(val)
+    cg = m.ConjugateGradient(A).setTolerance(1e-8).set_path(1)
+    x = cg.solve(torch.from_numpy(b.astype(np.float64)).to(cuda)).cpu().numpy()
+    assert np.all(cg.system_stats()["status"] == 0)
+    assert np.all(_residuals(off, row_ptr, col, val, b, x) <= 1.1e-8)
