@@ -44,6 +44,7 @@ struct alignas(16) OcScratch {
     VT redB[2 * kOcWarps];
     int slot;
 };
+static_assert(sizeof(OcScratch<double>) <= kOnchipStatic64, "");
 
 // Solves the work items [t.lo, t.hi) until none is left. T threads (and, OC_CLUSTER,
 // the cluster's CTAs) per system; H: virtual threads a thread plays (FP32; 1

@@ -34,7 +34,7 @@ struct alignas(16) MixScratch {
     int guard[3];   // progress guard of BF16 inner values (k_mixed_fast)
 };
 constexpr int kMixGroupScratch = (static_cast<int>(sizeof(MixScratch)) + 15) / 16 * 16;
-static_assert(kMixGroupScratch <= kOnchipMixScratch, "");
+static_assert(kMixGroupScratch <= kOnchipMixScratch && sizeof(MixScratch) <= kOnchipStaticMix256, "");
 
 // Solves the work items [t.lo, t.hi) until none is left, T threads per system,
 // H virtual threads per thread. sm: the group's dynamic shared memory.

@@ -38,6 +38,9 @@ constexpr int kOnchipMixTinyRows = 4096;   // above: 512 threads
 
 constexpr int kOnchipGroupScratch = 544;   // shared memory of a group's sums (FP32 launch)
 constexpr int kOnchipMixScratch = 1056;    // the same, mixed solve
+// Static shared memory of a CTA (the kernels' files assert it)
+constexpr int kOnchipStatic64 = 2064;      // k_onchip with FP64 vectors
+constexpr int kOnchipStaticMix256 = 2048;  // k_onchip_mixed256 (at most)
 
 // Row slots per thread of a system of n rows (a multiple of two, see the kernel).
 CMCG_HD inline int onchip_slots(int n, int threads, int ctas) {
@@ -69,8 +72,10 @@ inline bool onchip_halo_ok(const OnchipForm& f, int n, int reach) {
 }
 
 // Dynamic shared memory of a CTA when per_sm of them share an SM: 228 KB, of
-// which every CTA takes 1 KB for the system and less than 2 KB of static arrays.
-inline size_t onchip_smem_limit(int per_sm) { return static_cast<size_t>(228 * 1024 / per_sm) - 3 * 1024; }
+// which every CTA takes 1 KB for the system and its static arrays.
+inline size_t onchip_smem_limit(int per_sm, int static_bytes) {
+    return static_cast<size_t>(228 * 1024 / per_sm - 1024 - static_bytes);
+}
 // In the launches with FP32 vectors the systems share one CTA's memory, whose
 // static arrays are below 1 KB (plain) and 1.1 KB (mixed); a group of its threads
 // keeps its scratch in its part.
@@ -124,7 +129,8 @@ std::vector<OnchipTier> onchip_tiers(const OnchipBatch& b, const OnchipForm (&fo
         }
         const size_t s = onchip_smem<VT>(f, rows, b.nd, b.margin, b.val_bytes);
         const bool whole = sizeof(VT) == 8 || (b.mixed && f.threads == 256);   // CTAs of this form share the SM, not a CTA's part
-        const size_t limit = whole ? onchip_smem_limit(f.per_sm) : onchip_smem_limit32(f.per_sm, b.mixed);
+        const size_t limit = whole ? onchip_smem_limit(f.per_sm, sizeof(VT) == 8 ? kOnchipStatic64 : kOnchipStaticMix256)
+                                   : onchip_smem_limit32(f.per_sm, b.mixed);
         return s > 0 && s <= limit && onchip_halo_ok<VT>(f, rows, reach);
     };
     int32_t lo = b.first;

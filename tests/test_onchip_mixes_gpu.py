@@ -57,6 +57,8 @@ MIXES = {"long_grid": [_square(100)] * 10 + [_grid(2200, 2)] + [_square(58)] * 2
          "band": [_square(128)] * 10 + [(5000, (1, 3500))],
          "band_alone": [(5000, (1, 2499)), (4100, (3, 2100)), (9000, (1, 3000)), (12000, (7, 3071))],
          "wide": [_square(64)] * 150 + [_grid(3000, 3), _grid(1025, 15), _square(20)],
+         # (values, p and halo of an FP64 cluster at the shared memory's limit)
+         "halo_2110": [_grid(2110, 7)] * 20 + [_grid(2109, 7)] * 130,
          "small": [_grid(700, 2), _grid(2, 700), _square(31), (50, (1,)), (3, (2,))] * 40}
 
 

@@ -66,6 +66,16 @@ def _check(kind, systems, nd, val_bytes, ob, first, tiers):
     assert tiers[0]["lo"] == first * ob and tiers[-1]["hi"] == len(systems) * ob
     assert all(a["hi"] == b["lo"] for a, b in zip(tiers, tiers[1:]))
     for t in tiers:
+        # 227 KB of a CTA and 228 KB of an SM hold the dynamic and the static arrays
+        # and 1 KB per CTA for the system
+        if kind == 1 or (kind == 2 and t["threads"] == 256):
+            static = 2 * 128 * 8 + 16 if kind == 1 else 1040
+            assert t["smem"] + static <= 227 * 1024 and t["per_sm"] * (t["smem"] + static + 1024) <= 228 * 1024, t
+        else:   # groups share one CTA's memory, each with its scratch before its part
+            scratch, static = (544, 528) if kind == 0 else (1056, 1040)
+            part = -(-t["smem"] // 16) * 16 + (scratch if t["per_sm"] > 1 else 0)
+            assert -(-part * t["per_sm"] // 64) * 64 + static <= 227 * 1024, t
+    for t in tiers:
         per = t["threads"] * t["ctas"]
         for n, reach in systems[t["lo"] // ob:t["hi"] // ob]:
             nk = (-(-n // per) + 1) // 2 * 2
