@@ -169,8 +169,11 @@ cmcg_status ensure_dia(cmcg_pattern p) {
         const int32_t* o = off.data() + s * kDiaMax;
         for (int64_t r = ro[s]; r < ro[s + 1]; ++r) {
             const int64_t i = r - ro[s];
+            uint32_t seen = 0;
             for (int32_t k = rp[r]; k < rp[r + 1]; ++k) {
                 const int32_t d = static_cast<int32_t>(std::find(o, o + nd[s], static_cast<int32_t>(ci[k] - r)) - o);
+                if (seen >> d & 1) return CMCG_OK;   // two entries of one place add up: no slot for both
+                seen |= 1u << d;
                 pos[k] = static_cast<int32_t>(base[s] + B * ((i / B) * nd_alloc + d) + i % B);
             }
         }

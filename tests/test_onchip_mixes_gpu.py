@@ -75,3 +75,28 @@ def test_fp64_mixed_shapes(cuda, name, values):
     x = cg.solve(torch.from_numpy(b.astype(np.float64)).to(cuda)).cpu().numpy()
     assert np.all(cg.system_stats()["status"] == 0)
     assert np.all(_residuals(off, row_ptr, col, val, b, x) <= 1.1e-8)
+
+
+# one system on each path that reads stencil patterns in the diagonal layout, and a batch
+@pytest.mark.parametrize("systems,path", [([_square(31)] * 160, 0), ([_square(64)], 0), ([_square(100)], 0),
+                                          ([_square(400)], 0), ([_square(40)], 2)])
+@pytest.mark.parametrize("kind", ["fp32", "fp64", "mixed"])
+def test_repeated_entries_add_up(cuda, systems, path, kind):
+    # every entry stored as two (1/4 and 3/4 of it), which a product adds up
+    m = cm()
+    off, row_ptr, col, val, b = _pack(systems, 5)
+    n = b.size
+    quarter = (val * np.float32(0.25)).astype(np.float32)
+    v2 = np.stack([quarter, val - quarter], 1).ravel()
+    p = m.SparsityPattern.csr(n, n, row_ptr * 2, np.repeat(col, 2))
+    if len(systems) > 1:
+        p.set_systems(off)
+    dt = torch.float64 if kind == "fp64" else torch.float32
+    A = m.SparseMatrix(p, dtype=dt).setData(v2)
+    bt = torch.from_numpy(b).to(cuda).to(torch.float32 if kind == "fp32" else torch.float64)
+    cg = m.ConjugateGradient(A).setTolerance(1e-8 if kind == "fp64" else 1e-5).set_path(path)
+    x = (cg.solve_refined(bt, outer_tol=1e-10) if kind == "mixed" else cg.solve(bt)).cpu().numpy()
+    assert np.all(cg.system_stats()["status"] == 0)
+    # (FP32: the recursion drifts by at most 100 iterations of 2^-24 |A| |x| / |b| <= 50)
+    limit = {"fp32": 3.1e-4, "fp64": 1.1e-8, "mixed": 1.01e-10}[kind]
+    assert np.all(_residuals(off, row_ptr * 2, np.repeat(col, 2), v2, b, x) <= limit)
