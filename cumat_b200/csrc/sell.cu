@@ -121,72 +121,119 @@ void free_dia(DiaPlan& d) {
     d.plan_id = id;
 }
 
+namespace {
+
+// Slot of every entry in the diagonal layout; blocks x: systems, y: rows.
+__global__ void __launch_bounds__(256) k_dia_pos(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                                 const int32_t* __restrict__ row_off, int32_t n_sys,
+                                                 const int64_t* __restrict__ base, const int32_t* __restrict__ off,
+                                                 int32_t nd, int32_t* __restrict__ pos) {
+    constexpr int B = kDiaBlockRows;
+    for (int s = blockIdx.x; s < n_sys; s += gridDim.x) {
+        int o[kDiaMax];
+#pragma unroll
+        for (int d = 0; d < kDiaMax; ++d) o[d] = off[s * kDiaMax + d];
+        const int r0 = row_off[s], n = row_off[s + 1] - r0;
+        const int64_t b = base[s];
+        for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x) {
+            const int64_t row = b + static_cast<int64_t>(B) * (i / B) * nd + i % B;
+            for (int k = rp[r0 + i]; k < rp[r0 + i + 1]; ++k) {
+                // the first match: unused offsets are 0 and stand behind the system's own
+                const int diff = ci[k] - (r0 + i);
+                int at = 0;
+#pragma unroll
+                for (int d = kDiaMax - 1; d >= 0; --d)
+                    if (o[d] == diff) at = d;
+                pos[k] = static_cast<int32_t>(row + static_cast<int64_t>(B) * at);
+            }
+        }
+    }
+}
+
+}  // namespace
+
+// The offsets are found on the host, in one pass over the entries, the entries'
+// slots on the device. With the slots found on the host too (a second pass and an upload
+// of 4 bytes per entry) and a search per entry, the first FP32 solve of 300 systems of
+// 16^2 .. 31^2 rows took 4.05 ms and of 512 systems of 32^2 .. 128^2 rows 114 ms, longer
+// than on the sliced layout (2.3 and 109 ms); so 0.82 and 15.6 ms, of which the solve
+// is 0.32 and 4.2.
 cmcg_status ensure_dia(cmcg_pattern p) {
     DiaPlan& D = p->dia;
     if (p->format != CMCG_CSR || D.built) return CMCG_OK;
     D.built = true;   // a failed or inapplicable plan is not retried until the systems change
-    const auto& rp = p->h_row_ptr;
-    const auto& ci = p->h_col;
+    const int32_t* rp = p->h_row_ptr.data();
+    const int32_t* ci = p->h_col.data();
     const auto& ro = p->row_off;
     const int64_t n_sys = static_cast<int64_t>(ro.size()) - 1;
     std::vector<int32_t> off(static_cast<size_t>(n_sys) * kDiaMax, 0);
     std::vector<int64_t> base(n_sys);
-    std::vector<int32_t> nd(n_sys), reach(n_sys, 0);
-    int64_t slots = 0;
+    std::vector<int32_t> reach(n_sys, 0);
     int32_t max_nd = 0, margin = 0;
     for (int64_t s = 0; s < n_sys; ++s) {
-        std::vector<int32_t> o;
+        int32_t o[kDiaMax];   // the system's offsets, ascending
+        int32_t nd = 0;
         for (int64_t r = ro[s]; r < ro[s + 1]; ++r) {
-            for (int32_t k = rp[r]; k < rp[r + 1]; ++k) {
-                const int32_t d = static_cast<int32_t>(ci[k] - r);
-                if (std::find(o.begin(), o.end(), d) == o.end()) {
-                    if (static_cast<int>(o.size()) == kDiaMax) return CMCG_OK;   // not diagonal-shaped: D.ok stays false
-                    o.push_back(d);
+            const int32_t k0 = rp[r], k1 = rp[r + 1];
+            if (k1 - k0 == nd) {   // most rows: exactly the offsets found so far
+                int32_t other = 0;
+                for (int32_t d = 0; d < nd; ++d) other |= (ci[k0 + d] - static_cast<int32_t>(r)) ^ o[d];
+                if (other == 0) continue;
+            }
+            uint32_t seen = 0;   // offsets of this row
+            int32_t d = 0;
+            for (int32_t k = k0; k < k1; ++k) {
+                const int32_t diff = static_cast<int32_t>(ci[k] - r);
+                // columns mostly ascend: go on from the last entry's offset
+                if (d > 0 && o[d - 1] >= diff) d = 0;
+                while (d < nd && o[d] < diff) ++d;
+                if (d == nd || o[d] != diff) {
+                    if (nd == kDiaMax) return CMCG_OK;   // not diagonal-shaped: D.ok stays false
+                    std::copy_backward(o + d, o + nd, o + nd + 1);
+                    o[d] = diff;
+                    ++nd;
+                    const uint32_t below = seen & ((1u << d) - 1);
+                    seen = below | (seen - below) << 1;
+                } else if (seen >> d & 1) {
+                    return CMCG_OK;   // two entries of one place add up: no slot for both
                 }
+                seen |= 1u << d;
+                ++d;
             }
         }
-        std::sort(o.begin(), o.end());
-        for (size_t j = 0; j < o.size(); ++j) {
-            off[static_cast<size_t>(s) * kDiaMax + j] = o[j];
-            reach[s] = std::max(reach[s], std::abs(o[j]));
-        }
+        std::copy(o, o + nd, off.begin() + s * kDiaMax);
+        if (nd > 0) reach[s] = std::max(std::abs(o[0]), std::abs(o[nd - 1]));
         margin = std::max(margin, reach[s]);
-        nd[s] = static_cast<int32_t>(o.size());
-        max_nd = std::max(max_nd, nd[s]);
+        max_nd = std::max(max_nd, nd);
     }
     // every system stores the same number of diagonals (5 or 7, the widths the
     // kernel is built for); unused ones hold zeros
     const int32_t nd_alloc = max_nd <= 5 ? 5 : max_nd <= 7 ? 7 : 0;
     if (nd_alloc == 0) return CMCG_OK;
     constexpr int64_t B = kDiaBlockRows;
+    int64_t slots = 0;
     for (int64_t s = 0; s < n_sys; ++s) {
         base[s] = slots;
         slots += static_cast<int64_t>(nd_alloc) * ((ro[s + 1] - ro[s] + B - 1) / B) * B;
     }
     if (slots >= INT32_MAX) return CMCG_OK;
-    std::vector<int32_t> pos(static_cast<size_t>(p->nnz));
-    for (int64_t s = 0; s < n_sys; ++s) {
-        const int32_t* o = off.data() + s * kDiaMax;
-        for (int64_t r = ro[s]; r < ro[s + 1]; ++r) {
-            const int64_t i = r - ro[s];
-            uint32_t seen = 0;
-            for (int32_t k = rp[r]; k < rp[r + 1]; ++k) {
-                const int32_t d = static_cast<int32_t>(std::find(o, o + nd[s], static_cast<int32_t>(ci[k] - r)) - o);
-                if (seen >> d & 1) return CMCG_OK;   // two entries of one place add up: no slot for both
-                seen |= 1u << d;
-                pos[k] = static_cast<int32_t>(base[s] + B * ((i / B) * nd_alloc + d) + i % B);
-            }
-        }
-    }
-    auto up = [](void** dptr, const void* h, size_t bytes) -> cmcg_status {
-        CMCG_TRY(dev_alloc(dptr, std::max<size_t>(bytes, 16)));
-        if (bytes) CMCG_CUDA(cudaMemcpy(*dptr, h, bytes, cudaMemcpyHostToDevice));
+    cmcg_ctx ctx = p->ctx;
+    const auto build = [&]() -> cmcg_status {
+        CMCG_TRY(dev_alloc(reinterpret_cast<void**>(&D.d_pos), std::max<size_t>(static_cast<size_t>(p->nnz) * 4, 16)));
+        CMCG_TRY(dev_alloc(reinterpret_cast<void**>(&D.d_sys_base), base.size() * 8));
+        CMCG_TRY(dev_alloc(reinterpret_cast<void**>(&D.d_sys_off), off.size() * 4));
+        CMCG_CUDA(cudaMemcpyAsync(D.d_sys_base, base.data(), base.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+        CMCG_CUDA(cudaMemcpyAsync(D.d_sys_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+        const int64_t most = static_cast<int64_t>(ctx->sm_count) * 8;
+        const dim3 grid(static_cast<unsigned>(std::min(n_sys, most)), static_cast<unsigned>(std::max<int64_t>(1, most / n_sys)));
+        k_dia_pos<<<grid, 256, 0, ctx->stream>>>(p->d_row_ptr, p->d_col, p->d_row_off, static_cast<int32_t>(n_sys),
+                                                 D.d_sys_base, D.d_sys_off, nd_alloc, D.d_pos);
+        count_launch();
+        CMCG_CHECK_LAUNCH();
         return CMCG_OK;
     };
-    cmcg_status st;
-    if ((st = up(reinterpret_cast<void**>(&D.d_pos), pos.data(), pos.size() * 4)) != CMCG_OK ||
-        (st = up(reinterpret_cast<void**>(&D.d_sys_base), base.data(), base.size() * 8)) != CMCG_OK ||
-        (st = up(reinterpret_cast<void**>(&D.d_sys_off), off.data(), off.size() * 4)) != CMCG_OK) {
+    const cmcg_status st = build();
+    if (st != CMCG_OK) {
         free_dia(D);
         D.built = true;
         return st;

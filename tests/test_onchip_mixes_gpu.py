@@ -100,3 +100,31 @@ def test_repeated_entries_add_up(cuda, systems, path, kind):
     # (FP32: the recursion drifts by at most 100 iterations of 2^-24 |A| |x| / |b| <= 50)
     limit = {"fp32": 3.1e-4, "fp64": 1.1e-8, "mixed": 1.01e-10}[kind]
     assert np.all(_residuals(off, row_ptr * 2, np.repeat(col, 2), v2, b, x) <= limit)
+
+
+# rows either side of the layout's 1024-row blocks, systems of one and two rows, three
+# to seven offsets of a system, entries of a row in any order
+LAYOUT = [(1, ()), (2, (1,)), (1023, (1, 31)), (1024, (2,)), (1025, (1, 32, 33)), (2049, (1, 5, 1024)), (3000, (7,))]
+
+
+@pytest.mark.parametrize("order", ["ascending", "descending", "shuffled"])
+@pytest.mark.parametrize("kind", ["fp32", "fp64", "mixed", "product"])
+def test_entry_order_of_the_diagonal_layout(cuda, order, kind):
+    m = cm()
+    off, row_ptr, col, val, b = _pack(LAYOUT * 25, 3)
+    n = b.size
+    key = {"ascending": col, "descending": -col, "shuffled": np.random.RandomState(4).randint(0, 1 << 30, col.size)}[order]
+    perm = np.lexsort((key, np.repeat(np.arange(n), np.diff(row_ptr))))
+    col, val = col[perm], val[perm]
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p, dtype=torch.float64 if kind == "fp64" else torch.float32).setData(val)
+    bt = torch.from_numpy(b).to(cuda).to(torch.float32 if kind == "fp32" else torch.float64)
+    if kind == "product":   # the grid path's product in the layout: an iteration of it
+        cg = m.ConjugateGradient(A).setTolerance(1e-8).set_path(2)
+    else:
+        cg = m.ConjugateGradient(A).setTolerance(1e-5 if kind == "fp32" else 1e-8).set_path(1)
+    x = (cg.solve_refined(bt, outer_tol=1e-10) if kind == "mixed" else cg.solve(bt)).cpu().numpy()
+    assert np.all(cg.system_stats()["status"] == 0)
+    limit = {"fp32": 3.1e-4, "fp64": 1.1e-8, "mixed": 1.01e-10, "product": 1.1e-8}[kind]
+    assert np.all(_residuals(off, row_ptr, col, val, b, x) <= limit)
