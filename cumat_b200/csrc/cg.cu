@@ -3016,7 +3016,7 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
     a.st = s->st;
     CMCG_CUDA(cudaMemsetAsync(s->counters, 0, 8 * sizeof(int32_t), ctx->stream));
     if (s->refine_method == CMCG_REFINE_RELIABLE && FMT == CMCG_CSR && compact_ok(s)) {
-        CMCG_TRY(ensure_mix(s));
+        CMCG_TRY(ensure_scale(s));
         MixArgs<MI, MO> m{};
         m.rows = p->rows;
         m.n_sys = s->n_sys;
@@ -3026,8 +3026,6 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
         m.order = s->d_order;
         m.next = s->counters;
         m.c = compact_args(p);
-        m.vin = static_cast<const MI*>(s->mix_vals);
-        m.vin_stride = s->mix_stride;
         m.vout = static_cast<const MO*>(Ao->d_sell_vals);
         m.vout_stride = Ao->sell_stride;
         m.s = s->mix_s;
@@ -3058,6 +3056,12 @@ cmcg_status refined_persistent(cmcg_solver s, cmcg_matrix Ao, const double* b, i
             m.margin = p->dia.margin;
             m.dia_unit = s->dia_unit;
             nd = p->dia.max_nd;
+        } else {
+            // (the scaled values in the sliced layout: one copy of the batch more,
+            // which a solve on the diagonals does not read)
+            CMCG_TRY(ensure_mix(s));
+            m.vin = static_cast<const MI*>(s->mix_vals);
+            m.vin_stride = s->mix_stride;
         }
         // Three tiers by position in the size order: systems above
         // kMixSmallRows rows on 1024-thread CTAs (one per SM), then systems of

@@ -128,3 +128,33 @@ def test_entry_order_of_the_diagonal_layout(cuda, order, kind):
     assert np.all(cg.system_stats()["status"] == 0)
     limit = {"fp32": 3.1e-4, "fp64": 1.1e-8, "mixed": 1.01e-10, "product": 1.1e-8}[kind]
     assert np.all(_residuals(off, row_ptr, col, val, b, x) <= limit)
+
+
+@pytest.mark.parametrize("diagonals", [True, False])
+def test_value_uploads_rebuild_the_layouts_read(cuda, monkeypatch, diagonals):
+    # a mixed solve of systems either side of 8192 rows after a value upload: the scale,
+    # the sliced values (FP64 residual above 8192 rows), the scaled diagonals and the unit
+    # diagonal's flags, and the diagonals (FP64 residual below); on the sliced layout the
+    # scale and both sliced copies
+    m = cm()
+    if not diagonals:
+        monkeypatch.setenv("CUMAT_CG_DIA", "0")
+    off, row_ptr, col, val, b = _pack([_square(100), _square(50)], 5)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p).setData(val)
+    cg = m.ConjugateGradient(A).set_path(1)
+    bt = torch.from_numpy(b.astype(np.float64)).to(cuda)
+    launches = []
+    for scale in (None, 1.0, 3.0):
+        if scale is not None:
+            A.setData(val * np.float32(scale))
+        for again in (False, True):
+            before = m.launch_count()
+            x = cg.solve_refined(bt, outer_tol=1e-10).cpu().numpy()
+            launches.append(m.launch_count() - before)
+            assert np.all(_residuals(off, row_ptr, col, val * np.float32(scale or 1), b, x) <= 1.01e-10)
+    solve = 2
+    assert launches[1::2] == [solve] * 3
+    assert launches[2::2] == [solve + (5 if diagonals else 3)] * 2
