@@ -24,7 +24,8 @@
 // follows its last read of it, so single buffers are enough.
 //
 // Every wait is bounded: a poll that runs out sets the device error bit of the
-// grid barrier and the CTA leaves; the others run out the same way.
+// grid barrier and the CTA leaves; the others run out the same way, since what a
+// poll that ran out was to add is never published.
 #include <algorithm>
 #include <cstdlib>
 
@@ -100,6 +101,7 @@ struct ResidentArgs {
     uint64_t* words;   // kSumWords per sum
     int32_t* err;
     BarrierLimits lim;
+    int32_t partials[2];   // of a sum of one and of two values (n_virtual; a test waits for one more)
 };
 
 // Where this CTA and thread stand in the grid plan.
@@ -177,23 +179,24 @@ __device__ __forceinline__ bool resident_sum(VT (&v)[NV][kResPlay], SumScratch<V
     if (c >= 0 && c < C && c * static_cast<int>(gridDim.x) / C == static_cast<int>(blockIdx.x)) {
         const int t = c * 32 + lane;
         TaggedSum<VT, NV> part[3];
-        if (!resident_poll(m, [&] {
+        const bool got = resident_poll(m, [&] {
 #pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    part[k].load(t + k * kTile < nv, words + static_cast<int64_t>(t + k * kTile) * W, want);
-                return part[0].arrived(want) && part[1].arrived(want) && part[2].arrived(want);
-            }))
-            sc.fail = 1;
-        __syncwarp();
+            for (int k = 0; k < 3; ++k)
+                part[k].load(t + k * kTile < m.partials[NV - 1], words + static_cast<int64_t>(t + k * kTile) * W, want);
+            return part[0].arrived(want) && part[1].arrived(want) && part[2].arrived(want);
+        });
+        if (!got) sc.fail = 1;
+        // a total that lacks a partial is not published: the other CTAs run out too
+        const bool all = __all_sync(FULL, got);
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             VT s = VT(0);
 #pragma unroll
             for (int k = 0; k < 3; ++k)
-                if (t + k * kTile < nv) s += part[k].value(j);
+                if (t + k * kTile < m.partials[NV - 1]) s += part[k].value(j);
             r[j] = warp_sum(s);
         }
-        if (lane == 0) {
+        if (lane == 0 && all) {
             if constexpr (NV == 2) put_pair(fin + c * 4, r[0], r[1], tag);
             else put_value(fin + c * 4, r[0], tag);
         }
@@ -1026,7 +1029,8 @@ static cmcg_status resident_launch(const void* kern, A args, const ResidentGeom&
     if (const char* e = std::getenv("CUMAT_TEST_GRID_SPINS")) lim.spins = std::max(1LL, std::atoll(e));
     if (const char* e = std::getenv("CUMAT_TEST_GRID_EXTRA")) lim.extra = static_cast<unsigned>(std::max(0, std::atoi(e)));
     uint64_t* w = static_cast<uint64_t*>(ws);
-    ResidentArgs m{g, w, w + vec_bytes / 4 * even(g.n), err, lim};
+    ResidentArgs m{g, w, w + vec_bytes / 4 * even(g.n), err, lim, {g.n_virtual, g.n_virtual}};
+    if (std::getenv("CUMAT_TEST_GRID_PARTIAL")) m.partials[1] = std::min(g.n_virtual + 1, kResMaxVirtual);
     void* params[] = {&args, &m};
     CMCG_CUDA(cudaLaunchCooperativeKernel(kern, g.ctas, kResThreads, params, g.smem, st));
     *launched = true;

@@ -236,3 +236,28 @@ def test_tagged_word_waits_run_out(cuda, monkeypatch, side, path):
     monkeypatch.delenv("CUMAT_TEST_GRID_EXTRA")
     cg.solve(bt)
     assert ctx.device_errors() == 0 and cg.system_stats()["status"][0] == 0
+
+
+def test_a_sum_that_lacks_a_partial_is_not_accepted(cuda, monkeypatch):
+    # one combining warp waits for a partial that no CTA publishes: the total it could
+    # not form reaches no CTA, although the sum of what is there would converge
+    m = cm()
+    row_ptr, col, val, b = _system("2d", 400)
+    n = b.size
+    A = m.SparseMatrix(m.SparsityPattern.csr(n, n, row_ptr, col)).setData(val)
+    bt = torch.from_numpy(b).to(cuda)
+    ctx = m.Context.current()
+    ctx.device_errors()
+    # (r_1 = (4 - A) b / 4 here, about half of |b|: the first iteration converges)
+    cg = _solver(monkeypatch, A, NO_OTHER, True).setTolerance(0.95).set_path(2)
+    cg.solve(bt)
+    assert cg.system_stats()["status"][0] == 0 and cg.system_stats()["iterations"][0] == 0
+    monkeypatch.setenv("CUMAT_TEST_GRID_SPINS", "2000")
+    monkeypatch.setenv("CUMAT_TEST_GRID_PARTIAL", "1")
+    cg.solve(bt)
+    assert ctx.device_errors() & 2
+    assert cg.system_stats()["status"][0] != 0
+    monkeypatch.delenv("CUMAT_TEST_GRID_SPINS")
+    monkeypatch.delenv("CUMAT_TEST_GRID_PARTIAL")
+    cg.solve(bt)
+    assert ctx.device_errors() == 0 and cg.system_stats()["status"][0] == 0
