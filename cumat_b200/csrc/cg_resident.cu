@@ -145,8 +145,10 @@ __device__ __forceinline__ bool resident_poll(const ResidentArgs& m, F&& arrived
 // polled by one warp of every CTA. (With every CTA polling all partials the
 // waiting CTAs' polls delay the late ones' stores: 6 us a sum on 148 CTAs, against
 // 2 to 3 us for the two hops.) meanwhile() runs between the CTA's own
-// publication and the result. False when a poll ran out.
-template <typename VT, int NV, typename F>
+// publication and the result. False when a poll ran out. ORDER: what any thread
+// wrote to global memory before the sum, every thread reads after it (at L2): each
+// hop fences between the barrier or poll it follows and its own publication.
+template <typename VT, int NV, bool ORDER = false, typename F>
 __device__ __forceinline__ bool resident_sum(VT (&v)[NV][kResPlay], SumScratch<VT>& sc, const ResidentArgs& m,
                                              uint64_t* words, uint32_t tag, F&& meanwhile) {
     constexpr int W = kWords<VT> * NV, C = kTile / 32;
@@ -169,6 +171,7 @@ __device__ __forceinline__ bool resident_sum(VT (&v)[NV][kResPlay], SumScratch<V
         for (int j = 0; j < NV; ++j) r[j] = warp_sum(lane < C ? sc.warp[j][warp * C + lane] : VT(0));
         if (lane == 0 && vc < nv) {
             uint64_t* w = words + static_cast<int64_t>(vc) * W;
+            if constexpr (ORDER) __threadfence();
             if constexpr (NV == 2) put_pair(w, r[0], r[1], tag);
             else put_value(w, r[0], tag);
         }
@@ -186,6 +189,10 @@ __device__ __forceinline__ bool resident_sum(VT (&v)[NV][kResPlay], SumScratch<V
             return part[0].arrived(want) && part[1].arrived(want) && part[2].arrived(want);
         });
         if (!got) sc.fail = 1;
+        if constexpr (ORDER) {
+            __threadfence();
+            __syncwarp();
+        }
         // a total that lacks a partial is not published: the other CTAs run out too
         const bool all = __all_sync(FULL, got);
 #pragma unroll
@@ -197,6 +204,7 @@ __device__ __forceinline__ bool resident_sum(VT (&v)[NV][kResPlay], SumScratch<V
             r[j] = warp_sum(s);
         }
         if (lane == 0 && all) {
+            if constexpr (ORDER) __threadfence();
             if constexpr (NV == 2) put_pair(fin + c * 4, r[0], r[1], tag);
             else put_value(fin + c * 4, r[0], tag);
         }
@@ -209,6 +217,7 @@ __device__ __forceinline__ bool resident_sum(VT (&v)[NV][kResPlay], SumScratch<V
                 return part.arrived(want);
             }))
             sc.fail = 1;
+        if constexpr (ORDER) __threadfence();
         if (lane < C) {
 #pragma unroll
             for (int j = 0; j < NV; ++j) sc.fin[j][lane] = part.value(j);
@@ -863,10 +872,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_mixed(const __grid_
                 }
 #pragma unroll
             for (int h = 0; h < kResPlay; ++h) resident_fold(m.x64, m.s, m.xh, lo + at.a0[h], lo + at.a1[h]);
-            __threadfence();
             float none[1][kResPlay] = {};
-            if (!resident_sum<float, 1>(none, sc, ra, words3, tag, [] {})) break;
-            __threadfence();
+            if (!resident_sum<float, 1, /*ORDER=*/true>(none, sc, ra, words3, tag, [] {})) break;
             ++htag;
             double acc[2][kResPlay];
 #pragma unroll

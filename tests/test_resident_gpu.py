@@ -261,3 +261,24 @@ def test_a_sum_that_lacks_a_partial_is_not_accepted(cuda, monkeypatch):
     monkeypatch.delenv("CUMAT_TEST_GRID_PARTIAL")
     cg.solve(bt)
     assert ctx.device_errors() == 0 and cg.system_stats()["status"][0] == 0
+
+
+@pytest.mark.parametrize("kind,size", [("3d", 40), ("fv", 401), ("2d", 1000)])
+def test_resident_mixed_with_frequent_replacements(cuda, monkeypatch, kind, size):
+    # a replacement whenever the residual fell by a tenth: every one reads x entries that
+    # other CTAs have just folded
+    m = cm()
+    row_ptr, col, val, b = _system(kind, size)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    A, A64 = m.SparseMatrix(p).setData(val), m.SparseMatrix(p, dtype=torch.float64).setData(val)
+    bt = torch.from_numpy(b.astype(np.float64)).to(cuda)
+    out = []
+    for env in (NO_OTHER, GRAPH):
+        cg = _solver(monkeypatch, A, env, True).set_path(2).setMaxIterations(400).set_refinement(0, 0.9)
+        x = cg.solve_refined(bt, outer=A64, outer_tol=1e-11, max_outer=400).cpu().numpy()
+        out.append((x, cg.system_stats()))
+    assert out[0][1]["outer"][0] > 20
+    assert np.array_equal(out[0][0], out[1][0])
+    for k in ("iterations", "status", "outer", "error"):
+        assert out[0][1][k][0] == out[1][1][k][0], k
