@@ -1731,6 +1731,7 @@ struct cmcg_solver_s {
     // host copies: the systems in size order (d_order), their rows, and the
     // largest |offset| of each (filled from the diagonal plan on first use)
     std::vector<int32_t> order, order_rows, order_reach;
+    int test_tier_fail = -1;   // the tier whose launch a test lets fail (CUMAT_TEST_TIER_FAIL)
     // on-chip batched kernels where they apply (CUMAT_CG_ONCHIP=0 disables)
     bool onchip = true;
     bool use_smem = true;     // shared-memory-resident kernels where the systems fit
@@ -2100,7 +2101,8 @@ cmcg_status ensure_aux_stream(cmcg_solver s) {
 }
 
 // Launches `launch(j, stream)` for the nt tiers j side by side: the last on the
-// caller's stream, the others on the priority streams, joined back at the end.
+// caller's stream, the others on the priority streams, joined back at the end,
+// also after an error: the tiers that run still write x and the solver's state.
 template <typename F>
 cmcg_status fork_tiers(cmcg_solver s, int nt, F&& launch) {
     cmcg_ctx ctx = s->A->pat->ctx;
@@ -2108,18 +2110,30 @@ cmcg_status fork_tiers(cmcg_solver s, int nt, F&& launch) {
         CMCG_TRY(ensure_aux_stream(s));
         CMCG_CUDA(cudaEventRecord(s->ev_fork, ctx->stream));
     }
-    for (int j = 0; j < nt; ++j) {
+    int forked = 0;
+    const auto tier = [&](int j) -> cmcg_status {
         cudaStream_t st = (j == nt - 1) ? ctx->stream : s->aux_stream[j];
-        if (j < nt - 1) CMCG_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
+        if (j < nt - 1) {
+            CMCG_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
+            forked = j + 1;
+        }
+        if (j == s->test_tier_fail) return fail(CMCG_ERR_INTERNAL, "launch of a tier failed (CUMAT_TEST_TIER_FAIL)");
         CMCG_TRY(launch(j, st));
         CMCG_CHECK_LAUNCH();
         count_launch();
+        return CMCG_OK;
+    };
+    cmcg_status rc = CMCG_OK;
+    for (int j = 0; j < nt && rc == CMCG_OK; ++j) rc = tier(j);
+    for (int j = 0; j < forked; ++j) {
+        cudaError_t e = cudaEventRecord(s->ev_join[j], s->aux_stream[j]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, s->ev_join[j], 0);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(s->aux_stream[j]);
+            if (rc == CMCG_OK) rc = cuda_fail(e, "joining the tier streams", __FILE__, __LINE__);
+        }
     }
-    for (int j = 0; j < nt - 1; ++j) {
-        CMCG_CUDA(cudaEventRecord(s->ev_join[j], s->aux_stream[j]));
-        CMCG_CUDA(cudaStreamWaitEvent(ctx->stream, s->ev_join[j], 0));
-    }
-    return CMCG_OK;
+    return rc;
 }
 
 // Residual-replacement threshold of the reliable updates: the one set, else
@@ -3420,6 +3434,7 @@ cmcg_status cmcg_cg_create(cmcg_matrix A, int32_t precond, cmcg_solver* out) {
     if (const char* e = std::getenv("CUMAT_CG_SMALL")) s->mix_small = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_COOP")) s->coop = std::max(0, std::min(2, std::atoi(e)));
     if (const char* e = std::getenv("CUMAT_CG_CLUSTER")) s->cluster = std::atoi(e) != 0;
+    if (const char* e = std::getenv("CUMAT_TEST_TIER_FAIL")) s->test_tier_fail = std::atoi(e);
     if (const char* e = std::getenv("CUMAT_CG_ONCHIP")) s->onchip = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_WIDE")) s->wide = std::atoi(e) != 0;
     if (const char* e = std::getenv("CUMAT_CG_RESIDENT")) s->resident = std::atoi(e) != 0;

@@ -158,3 +158,31 @@ def test_value_uploads_rebuild_the_layouts_read(cuda, monkeypatch, diagonals):
     solve = 2
     assert launches[1::2] == [solve] * 3
     assert launches[2::2] == [solve + (5 if diagonals else 3)] * 2
+
+
+@pytest.mark.parametrize("kind", ["fp64", "mixed"])
+def test_a_failed_tier_launch_waits_for_the_others(cuda, monkeypatch, kind):
+    # the second launch of a solve of two forms fails: the call raises, and what follows
+    # on the caller's stream comes after the first launch, which still writes x
+    m = cm()
+    systems = [_square(110)] * 600 + [_square(40)] * 50
+    off, row_ptr, col, val, b = _pack(systems, 5)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p, dtype=torch.float64 if kind == "fp64" else torch.float32).setData(val)
+    bt = torch.from_numpy(b.astype(np.float64)).to(cuda)
+    solve = lambda cg, x: (cg.solve(bt, out=x) if kind == "fp64"  # noqa: E731
+                           else cg.solve_refined(bt, outer_tol=1e-8, out=x))
+    big = int(off[600])
+    want = solve(m.ConjugateGradient(A).setTolerance(1e-8), None).cpu().numpy()   # (all layouts in place)
+    monkeypatch.setenv("CUMAT_TEST_TIER_FAIL", "1")
+    cg = m.ConjugateGradient(A).setTolerance(1e-8)
+    monkeypatch.delenv("CUMAT_TEST_TIER_FAIL")
+    x = torch.full((n,), float("nan"), dtype=torch.float64, device=cuda)
+    for _ in range(2):
+        x.fill_(float("nan"))
+        with pytest.raises(m.CuMatError):
+            solve(cg, x)
+        got = x.cpu().numpy()
+        assert np.array_equal(got[:big], want[:big]) and np.all(np.isnan(got[big:]))
