@@ -2069,34 +2069,27 @@ inline int smem_rows(int32_t max_rows) { return (max_rows + 3) / 4 * 4; }
 constexpr size_t kMixSmallSmemLimit = 104 * 1024;
 constexpr size_t kMixTinySmemLimit = 50 * 1024;
 
-// Streams of descending priority (from the highest) and fork / join events, for
-// running the CTA tiers of a batched solve side by side (created on first use).
-// The handles are created into locals and kept only when every creation
-// succeeded (a partial set is destroyed), so a failure leaves the solver
-// without any and the next call tries again.
-cmcg_status ensure_aux_stream(cmcg_solver s) {
-    if (s->ev_fork) return CMCG_OK;
-    int least = 0, greatest = 0;
-    CMCG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    cudaStream_t st[kAuxStreams] = {};
-    cudaEvent_t ev[kAuxStreams + 1] = {};
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < kAuxStreams && e == cudaSuccess; ++k)
-        e = cudaStreamCreateWithPriority(&st[k], cudaStreamNonBlocking, std::min(least, greatest + k));
-    for (int k = 0; k <= kAuxStreams && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
-    if (e != cudaSuccess) {
-        for (auto x : st)
-            if (x) cudaStreamDestroy(x);
-        for (auto x : ev)
-            if (x) cudaEventDestroy(x);
-        cudaGetLastError();
-        return fail(CMCG_ERR_CUDA, std::string("creating the tier streams: ") + cudaGetErrorString(e));
+// The first n streams of descending priority (from the highest) with their join
+// events, and the fork event, for running the CTA tiers of a batched solve side by
+// side: created when a solve first has that many tiers (a mixed solve has up to
+// three, an FP64 solve up to six). A stream is kept only with its event, so that a
+// failure leaves whole pairs and the next call tries again.
+cmcg_status ensure_aux_streams(cmcg_solver s, int n) {
+    if (!s->ev_fork) CMCG_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
+    for (int k = 0; k < n; ++k) {
+        if (s->aux_stream[k]) continue;
+        int least = 0, greatest = 0;
+        CMCG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        cudaStream_t st = nullptr;
+        CMCG_CUDA(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, std::min(least, greatest + k)));
+        const cudaError_t e = cudaEventCreateWithFlags(&s->ev_join[k], cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            s->ev_join[k] = nullptr;
+            cudaStreamDestroy(st);
+            return cuda_fail(e, "creating the tier streams", __FILE__, __LINE__);
+        }
+        s->aux_stream[k] = st;
     }
-    for (int k = 0; k < kAuxStreams; ++k) {
-        s->aux_stream[k] = st[k];
-        s->ev_join[k] = ev[k];
-    }
-    s->ev_fork = ev[kAuxStreams];
     return CMCG_OK;
 }
 
@@ -2107,7 +2100,7 @@ template <typename F>
 cmcg_status fork_tiers(cmcg_solver s, int nt, F&& launch) {
     cmcg_ctx ctx = s->A->pat->ctx;
     if (nt > 1) {
-        CMCG_TRY(ensure_aux_stream(s));
+        CMCG_TRY(ensure_aux_streams(s, nt - 1));
         CMCG_CUDA(cudaEventRecord(s->ev_fork, ctx->stream));
     }
     int forked = 0;
