@@ -72,6 +72,7 @@ cmcg_status fail(cmcg_status code, const std::string& msg) {
 }
 
 cmcg_status cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
+    (void)cudaGetLastError();   // (reported here: not by the next call's launch check too)
     const char* base = std::strrchr(file, '/');
     g_last_error = std::string("CUDA error '") + cudaGetErrorString(e) + "' in " + what + " (" +
                    (base ? base + 1 : file) + ":" + std::to_string(line) + ")";

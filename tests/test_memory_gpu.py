@@ -70,3 +70,19 @@ def test_reductions_and_products_after_dirty_blocks(cuda):
         B = m.SparseMatrix(m.SparsityPattern.csr(pr.n, pr.n, pr.row_ptr, pr.col)).setData(pr.val)
         assert np.array_equal(B.transposed_product(v).cpu().numpy(), y0)
         del B
+
+
+def test_an_error_is_reported_once(cuda):
+    # an allocation no device can hold fails; the calls after it do not report it again
+    import ctypes as C
+    import cumat_b200 as m
+    from cumat_b200 import _native as N
+    ctx = m.Context.current()
+    A = m.SparseMatrix(m.SparsityPattern.csr(2, 2, np.array([0, 1, 2], np.int32), np.array([0, 1], np.int32)))
+    for _ in range(2):
+        p = C.c_void_p()
+        with pytest.raises(m.CuMatError):
+            N.call("cmcg_device_alloc", ctx.handle, 1 << 50, C.byref(p))
+        A.setData(np.array([2.0, 4.0], np.float32))
+        x = m.ConjugateGradient(A).solve(torch.ones(2, device=cuda))
+        assert np.allclose(x.cpu().numpy(), [0.5, 0.25])
