@@ -186,3 +186,83 @@ def test_a_failed_tier_launch_waits_for_the_others(cuda, monkeypatch, kind):
             solve(cg, x)
         got = x.cpu().numpy()
         assert np.array_equal(got[:big], want[:big]) and np.all(np.isnan(got[big:]))
+
+
+@pytest.mark.parametrize("values", [torch.float64, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", sorted(MIXES))
+def test_fp64_guess_and_preconditioner(cuda, monkeypatch, name, values):
+    # against the kernels the forms stand in for: the statuses, the iteration counts (the
+    # sums differ in their order) and the true residual of every combination
+    m = cm()
+    off, row_ptr, col, val, b = _pack(MIXES[name], 13)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p, dtype=values).setData(val)
+    val = A.getData().astype(np.float64).reshape(-1)   # (BF16: as stored)
+    bt = torch.from_numpy(b.astype(np.float64)).to(cuda)
+    guess = torch.from_numpy(P.uniform(17, n).astype(np.float64)).to(cuda)
+    for precond in (m.DiagonalPreconditioner, m.IdentityPreconditioner):
+        for g in (None, guess):
+            stats = []
+            for onchip in ("1", "0"):
+                monkeypatch.setenv("CUMAT_CG_ONCHIP", onchip)
+                cg = m.ConjugateGradient(A, precond).setTolerance(1e-8).set_path(1)
+                x = cg.solveWithGuess(bt, g).cpu().numpy()
+                stats.append(cg.system_stats())
+                ok = stats[-1]["status"] == 0
+                assert np.all(_residuals(off, row_ptr, col, val, b, x)[ok] <= 1.1e-8)
+            assert np.array_equal(stats[0]["status"], stats[1]["status"])
+            if values != torch.bfloat16:   # (rounded to 8 bits the matrices may lose definiteness)
+                assert np.all(stats[0]["status"] == 0)
+                assert np.all(np.abs(stats[0]["iterations"] - stats[1]["iterations"]) <= 2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("rhs", ["one", "each"])
+def test_value_sets_on_one_pattern(cuda, dtype, rhs):
+    # several value sets on one packed pattern of mixed shapes, one right-hand side for all
+    # or one each, with a guess
+    m = cm()
+    systems = [_square(100), _grid(700, 4), _square(58), (5000, (1, 1400)), _square(12)]
+    off, row_ptr, col, val, b = _pack(systems, 7)
+    n, B = b.size, 30
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    vals = np.stack([val * np.float32(1 + 0.05 * i) for i in range(B)])
+    bs = np.stack([P.uniform(i, n) for i in range(B)]) if rhs == "each" else b
+    A = m.SparseMatrix(p, dtype=dtype, batches=B).setData(vals)
+    tol = 1e-8 if dtype == torch.float64 else 1e-5
+    cg = m.ConjugateGradient(A).setTolerance(tol).set_path(1)
+    guess = torch.from_numpy(np.stack([P.uniform(50 + i, n) for i in range(B)])).to(cuda).to(dtype)
+    for g in (None, guess):
+        x = cg.solveWithGuess(torch.from_numpy(bs).to(cuda).to(dtype), g).cpu().numpy()
+        assert np.all(cg.system_stats()["status"] == 0)
+        for i in range(B):
+            res = _residuals(off, row_ptr, col, vals[i], bs[i] if rhs == "each" else b, x[i])
+            # (FP32: the recursion drifts by at most 100 iterations of 2^-24 |A| |x| / |b| <= 50)
+            assert np.all(res <= (1.1e-8 if dtype == torch.float64 else 3.1e-4))
+
+
+@pytest.mark.parametrize("name", sorted(MIXES))
+def test_fp32_and_mixed_shapes_equal_persistent(cuda, monkeypatch, name):
+    # these keep the order of sums of the kernels they stand in for: bit for bit
+    m = cm()
+    off, row_ptr, col, val, b = _pack(MIXES[name], 19)
+    n = b.size
+    p = m.SparsityPattern.csr(n, n, row_ptr, col)
+    p.set_systems(off)
+    A = m.SparseMatrix(p).setData(val)
+    bt = torch.from_numpy(b).to(cuda)
+    for mixed in (False, True):
+        out = []
+        for onchip in ("1", "0"):
+            monkeypatch.setenv("CUMAT_CG_ONCHIP", onchip)
+            cg = m.ConjugateGradient(A).setTolerance(1e-5).set_path(1)
+            x = cg.solve_refined(bt.double(), outer_tol=1e-10) if mixed else cg.solve(bt)
+            out.append((x.cpu().numpy(), cg.system_stats()))
+        assert np.array_equal(out[0][0], out[1][0])
+        for k in ("iterations", "status", "error"):
+            assert np.array_equal(out[0][1][k], out[1][1][k]), k
+        if mixed:
+            assert np.all(_residuals(off, row_ptr, col, val, b, out[0][0]) <= 1.01e-10)
