@@ -1020,7 +1020,7 @@ def run_profile_case(case: str):
                 to 1e-10 (k_onchip, a launch per form)
     vectors     dot, squared norm, linear combination of 4 terms and the
                 sampled outer product on n = 64 Mi entries (k_dot, k_lincomb,
-                k_sddmm_csr on the 8192^2 Poisson pattern)
+                k_sddmm_csr_rows on the 8192^2 Poisson pattern)
     spmv_big    CSR and ELLPACK products on the 8192^2 Poisson matrix (3 each)
     reduce      sums of 2^28 FP32 values along rows, columns, batches (1024
                 each) and over all axes, kernel choice included (k_red_*)

@@ -1744,7 +1744,7 @@ struct cmcg_solver_s {
     bool cluster = true;
     // chip-resident solve of the grid path where it applies (CUMAT_CG_RESIDENT=0 disables)
     bool resident = true;
-    // one system of the cluster solve spread over all SMs (CUMAT_CG_WIDE=0 disables)
+    // one system of the cluster solve spread over more SMs (CUMAT_CG_WIDE=0 disables)
     bool wide = true;
     void* res_ws = nullptr;   size_t res_ws_bytes = 0;
     // grid path: the product forms p_k (-1: by the batch's vector bytes against
@@ -2657,7 +2657,7 @@ cmcg_status resident_geom(cmcg_solver s, int32_t ob, size_t val_bytes, size_t ve
 // one cooperative launch (cg_resident.cu) after the grid path's init kernels.
 // *done = false leaves the solve to the graph loop. Faster wherever it fits, us
 // per iteration here against the graph loop: FP32 Poisson 400^2 7.2 / 21.2, 1024^2
-// 10.6 / 26.3, 1023^2 14.7 / 31.2; 3-D 7-point 64^3 9.3 / 22.5, 96^3 20.7 / 28.4;
+// 9.8 / 25, 1023^2 14.7 / 31.2; 3-D 7-point 64^3 9.3 / 22.5, 96^3 20.7 / 28.4;
 // FP64 300^2 9.5 / 22.0, 720^2 12.8 / 31.5.
 template <typename VT, typename MT, int FMT>
 cmcg_status run_resident(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
@@ -2739,7 +2739,7 @@ cmcg_status run_cluster(cmcg_solver s, SolveArgs<VT, MT>& a, bool* done) {
         CMCG_CUDA(cudaMemsetAsync(s->st.bb, 0, sizeof(double), ctx->stream));
         CMCG_TRY((wide_cg_launch<VT, MT>(c, lg, ctas, nd, ctx->sm_count, s->res_ws, ctx->d_err, ctx->stream, &launched)));
         if (launched) {
-            if (log_on(2)) log_msg(2, "solve spread over all SMs: %d rows, %d rows per thread", c.rows, 1 << (lg - 10));
+            if (log_on(2)) log_msg(2, "solve spread over the SMs: %d rows, %d rows per thread", c.rows, 1 << (lg - 10));
             count_launch();
             *done = true;
             return CMCG_OK;

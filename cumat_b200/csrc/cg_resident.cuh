@@ -6,7 +6,7 @@
 
 namespace cmcg {
 
-constexpr int kResThreads = 512;       // 128 registers a thread: no spills with two quads
+constexpr int kResThreads = 512;       // 128 registers a thread (plain FP32, two quads: 128 .. 336 bytes of spills)
 constexpr int kResVirtual = 4;         // virtual 256-thread CTAs (of the grid plan) per CTA
 constexpr int kResMaxWindows = 8;
 constexpr int kResMaxVirtual = 3 * kTile;   // partial sums one combining thread may add: 3

@@ -1,4 +1,4 @@
-// PCG of one mid-size stencil system spread over every SM with all its state in
+// PCG of one mid-size stencil system spread over many SMs with all its state in
 // registers: one cooperative launch for the whole solve.
 //
 // The cluster solve (cg_cluster.cu) holds such a system in the shared memory of
@@ -7,9 +7,10 @@
 // run anywhere: unit (k, w) is warp w of cluster CTA k, its lane l owns the rows
 // k 2^lg + 1024 j + 32 w + l of the system, j < J = 2^lg / 1024, and keeps their
 // p, r, x, inverse diagonal and matrix values, and the p entries its products
-// gather, in registers. An SM holds eight units, so an iteration is
-// bound by latency: two rounds through L2, one per reduction (published and
-// polled as tagged words, tagged.cuh). The z entries a neighbour gathers are
+// gather, in registers. A CTA holds eight units and an SM one CTA: 40 SMs at 100^2, 44
+// at 300^2, 64 at most. An iteration is bound by latency (300^2: 21 % of the issue slots
+// of its SMs used): two rounds through L2, one per reduction (published and polled as tagged
+// words, tagged.cuh). The z entries a neighbour gathers are
 // published before the second reduction; every reader forms p = z + beta p for
 // itself.
 //
@@ -74,8 +75,7 @@ __device__ __forceinline__ void wide_publish(VT (&v)[NV], const WideArgs& a, int
 
 // False when a poll ran out.
 template <typename VT, int NV>
-__device__ __forceinline__ bool wide_collect(VT (&v)[NV], const WideArgs& a, WideScratch& sc, int unit, int set,
-                                             uint32_t tag, uint32_t want) {
+__device__ __forceinline__ bool wide_collect(VT (&v)[NV], const WideArgs& a, WideScratch& sc, int set, uint32_t want) {
     constexpr int S = NV * kWords<VT>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     uint64_t* const words = a.words + set * kWideWords;
@@ -113,7 +113,7 @@ template <typename VT, int NV>
 __device__ __forceinline__ bool wide_sum(VT (&v)[NV], const WideArgs& a, WideScratch& sc, int unit, int set,
                                          uint32_t tag, uint32_t want) {
     wide_publish<VT, NV>(v, a, unit, set, tag);
-    return wide_collect<VT, NV>(v, a, sc, unit, set, tag, want);
+    return wide_collect<VT, NV>(v, a, sc, set, want);
 }
 
 // The z words of the rows other threads own, read into zn (bit j ND + d of
@@ -122,7 +122,8 @@ __device__ __forceinline__ bool wide_sum(VT (&v)[NV], const WideArgs& a, WideScr
 template <typename VT, int ND, int J>
 __device__ __forceinline__ void wide_gather(VT (&zn)[J][ND], uint64_t need, const WideArgs& a, WideScratch& sc,
                                             const int (&off)[ND], int row0, int set, uint32_t want) {
-    // (at most 28 words in flight: the registers of a 128-thread CTA)
+    // (at most 28 words in flight: a 256-thread CTA has 255 registers a thread. The widest
+    // forms with seven diagonals spill, FP32 J = 8 504 bytes and FP64 J = 4 580; no other does)
     constexpr int JG = J * ND * kWords<VT> <= 28 ? J : J * ND * kWords<VT> <= 56 ? J / 2 : J / 4;
 #pragma unroll
     for (int j0 = 0; j0 < J; j0 += JG) {
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(32 * kWideMaxWarps, 1) k_wide_cg(const __grid_
         // (the neighbours' z arrives while the sum is under way)
         VT zn[J][ND];
         wide_gather<VT, ND, J>(zn, need, w, sc, off, row0, 1, want);
-        if (!wide_collect<VT, 2>(s2, w, sc, unit, 1, tag, want)) break;
+        if (!wide_collect<VT, 2>(s2, w, sc, 1, want)) break;
         rr = s2[0];
         if (!finite_(rr) || !finite_(s2[1])) { status = CMCG_SOLVE_NON_FINITE; break; }
         if (rr < thr) { status = CMCG_SOLVE_CONVERGED; break; }

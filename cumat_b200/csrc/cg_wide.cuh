@@ -1,4 +1,4 @@
-// One mid-size stencil system spread over all SMs (cg_wide.cu).
+// One mid-size stencil system spread over up to 64 SMs (cg_wide.cu).
 #pragma once
 
 #include "cg_grid.cuh"
